@@ -847,13 +847,20 @@ struct Amr3 {
     FArr3 val{valp, nvar, nrow, ncol, nfil};
     const double hxmarg = hx * 0.01, hymarg = hy * 0.01, hzmarg = hz * 0.01;
     if (xperdom && yperdom && zperdom) return;
+    // A periodic piece (prefilrecur) may lie wholly beyond a wall or extrapolation face: its
+    // array then has no interior cell to copy from. Those cells keep what they hold; the
+    // patch's own call sets them once the pieces are in place.
+    auto at = [](int s, int n) { return s >= 1 && s <= n; };
     auto chk = [&](int code) { if (code == 0) throw std::runtime_error("user boundary conditions are not provided"); };
     if (xlo_p < xlower - hxmarg) {
       const int nxl = (int)((xlower + hxmarg - xlo_p) / hx);
       chk(mthbc[1]);
       if (mthbc[1] == 1 || mthbc[1] == 3) {
         for (int k = 1; k <= nfil; ++k) for (int j = 1; j <= ncol; ++j) for (int i = 1; i <= nxl; ++i)
-          for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, mthbc[1] == 1 ? nxl + 1 : 2 * nxl + 1 - i, j, k);
+          {
+            const int s = mthbc[1] == 1 ? nxl + 1 : 2 * nxl + 1 - i;
+            if (at(s, nrow)) for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, s, j, k);
+          }
         if (mthbc[1] == 3)
           for (int k = 1; k <= nfil; ++k) for (int j = 1; j <= ncol; ++j) for (int i = 1; i <= nxl; ++i) val(2, i, j, k) = -val(2, i, j, k);
       }
@@ -864,7 +871,10 @@ struct Amr3 {
       chk(mthbc[2]);
       if (mthbc[2] == 1 || mthbc[2] == 3) {
         for (int k = 1; k <= nfil; ++k) for (int i = ibeg; i <= nrow; ++i) for (int j = 1; j <= ncol; ++j)
-          for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, mthbc[2] == 1 ? ibeg - 1 : 2 * ibeg - 1 - i, j, k);
+          {
+            const int s = mthbc[2] == 1 ? ibeg - 1 : 2 * ibeg - 1 - i;
+            if (at(s, nrow)) for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, s, j, k);
+          }
         if (mthbc[2] == 3)
           for (int k = 1; k <= nfil; ++k) for (int i = ibeg; i <= nrow; ++i) for (int j = 1; j <= ncol; ++j) val(2, i, j, k) = -val(2, i, j, k);
       }
@@ -874,7 +884,10 @@ struct Amr3 {
       chk(mthbc[3]);
       if (mthbc[3] == 1 || mthbc[3] == 3) {
         for (int k = 1; k <= nfil; ++k) for (int j = 1; j <= nyl; ++j) for (int i = 1; i <= nrow; ++i)
-          for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, i, mthbc[3] == 1 ? nyl + 1 : 2 * nyl + 1 - j, k);
+          {
+            const int s = mthbc[3] == 1 ? nyl + 1 : 2 * nyl + 1 - j;
+            if (at(s, ncol)) for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, i, s, k);
+          }
         if (mthbc[3] == 3)
           for (int k = 1; k <= nfil; ++k) for (int j = 1; j <= nyl; ++j) for (int i = 1; i <= nrow; ++i) val(3, i, j, k) = -val(3, i, j, k);
       }
@@ -885,7 +898,10 @@ struct Amr3 {
       chk(mthbc[4]);
       if (mthbc[4] == 1 || mthbc[4] == 3) {
         for (int k = 1; k <= nfil; ++k) for (int j = jbeg; j <= ncol; ++j) for (int i = 1; i <= nrow; ++i)
-          for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, i, mthbc[4] == 1 ? jbeg - 1 : 2 * jbeg - 1 - j, k);
+          {
+            const int s = mthbc[4] == 1 ? jbeg - 1 : 2 * jbeg - 1 - j;
+            if (at(s, ncol)) for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, i, s, k);
+          }
         if (mthbc[4] == 3)
           for (int k = 1; k <= nfil; ++k) for (int j = jbeg; j <= ncol; ++j) for (int i = 1; i <= nrow; ++i) val(3, i, j, k) = -val(3, i, j, k);
       }
@@ -895,7 +911,10 @@ struct Amr3 {
       chk(mthbc[5]);
       if (mthbc[5] == 1 || mthbc[5] == 3) {
         for (int k = 1; k <= nzl; ++k) for (int j = 1; j <= ncol; ++j) for (int i = 1; i <= nrow; ++i)
-          for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, i, j, mthbc[5] == 1 ? nzl + 1 : 2 * nzl + 1 - k);
+          {
+            const int s = mthbc[5] == 1 ? nzl + 1 : 2 * nzl + 1 - k;
+            if (at(s, nfil)) for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, i, j, s);
+          }
         if (mthbc[5] == 3)
           for (int k = 1; k <= nzl; ++k) for (int j = 1; j <= ncol; ++j) for (int i = 1; i <= nrow; ++i) val(4, i, j, k) = -val(4, i, j, k);
       }
@@ -906,7 +925,10 @@ struct Amr3 {
       chk(mthbc[6]);
       if (mthbc[6] == 1 || mthbc[6] == 3) {
         for (int k = kbeg; k <= nfil; ++k) for (int j = 1; j <= ncol; ++j) for (int i = 1; i <= nrow; ++i)
-          for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, i, j, mthbc[6] == 1 ? kbeg - 1 : 2 * kbeg - 1 - k);
+          {
+            const int s = mthbc[6] == 1 ? kbeg - 1 : 2 * kbeg - 1 - k;
+            if (at(s, nfil)) for (int m = 1; m <= nvar; ++m) val(m, i, j, k) = val(m, i, j, s);
+          }
         if (mthbc[6] == 3)
           for (int k = kbeg; k <= nfil; ++k) for (int j = 1; j <= ncol; ++j) for (int i = 1; i <= nrow; ++i) val(4, i, j, k) = -val(4, i, j, k);
       }
