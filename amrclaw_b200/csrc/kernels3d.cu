@@ -1156,9 +1156,13 @@ __global__ void fill3_kernel(Fill3Args a) {
 // line[(g-1)*st]) set from the interior. code 1 copies cell s_ext into each; code 3 (wall)
 // mirrors cell refl-g into cell g and negates the normal momentum (neg). The sources of a
 // side never overlap its ghost cells, so every source is loaded before the first store.
+// A periodic piece may lie wholly beyond the face and hold no interior cell at all: a source
+// outside the line's n cells is not read, and the cell is set later, with its patch's own ghosts.
 template <class T>
-__device__ __forceinline__ void bc3_side(T* line, long long st, int lo, int hi, int code, int s_ext, int refl, bool neg) {
+__device__ __forceinline__ void bc3_side(T* line, long long st, int n_line, int lo, int hi, int code, int s_ext, int refl, bool neg) {
+  auto inside = [n_line](int s) { return s >= 1 && s <= n_line; };
   if (code == 1) {
+    if (!inside(s_ext)) return;
     const T x = line[(long long)(s_ext - 1) * st];
     for (int g = lo; g <= hi; ++g) line[(long long)(g - 1) * st] = x;
     return;
@@ -1169,13 +1173,14 @@ __device__ __forceinline__ void bc3_side(T* line, long long st, int lo, int hi, 
     T buf[MAXG];
 #pragma unroll
     for (int u = 0; u < MAXG; ++u)
-      if (u < n) buf[u] = line[(long long)(refl - (lo + u) - 1) * st];
+      if (u < n && inside(refl - (lo + u))) buf[u] = line[(long long)(refl - (lo + u) - 1) * st];
 #pragma unroll
     for (int u = 0; u < MAXG; ++u)
-      if (u < n) line[(long long)(lo + u - 1) * st] = neg ? -buf[u] : buf[u];
+      if (u < n && inside(refl - (lo + u))) line[(long long)(lo + u - 1) * st] = neg ? -buf[u] : buf[u];
     return;
   }
   for (int g = lo; g <= hi; ++g) {
+    if (!inside(refl - g)) continue;
     const T x = line[(long long)(refl - g - 1) * st];
     line[(long long)(g - 1) * st] = neg ? -x : x;
   }
@@ -1203,18 +1208,18 @@ __global__ void __launch_bounds__(128, 8) bc3_kernel(Bc3Args a) {
     T* base = v + m * plane;
     if constexpr (phase == 0) {
       T* line = base + (long long)l * nr;  // row (j,k) = (l % nc + 1, l / nc + 1)
-      if (o.nxl > 0 && (o.bxl == 1 || o.bxl == 3)) bc3_side(line, 1, 1, o.nxl, o.bxl, o.nxl + 1, 2 * o.nxl + 1, o.bxl == 3 && m == 1);
-      if (o.ibeg > 0 && (o.bxr == 1 || o.bxr == 3)) bc3_side(line, 1, o.ibeg, nr, o.bxr, o.ibeg - 1, 2 * o.ibeg - 1, o.bxr == 3 && m == 1);
+      if (o.nxl > 0 && (o.bxl == 1 || o.bxl == 3)) bc3_side(line, 1, nr, 1, o.nxl, o.bxl, o.nxl + 1, 2 * o.nxl + 1, o.bxl == 3 && m == 1);
+      if (o.ibeg > 0 && (o.bxr == 1 || o.bxr == 3)) bc3_side(line, 1, nr, o.ibeg, nr, o.bxr, o.ibeg - 1, 2 * o.ibeg - 1, o.bxr == 3 && m == 1);
     } else if constexpr (phase == 1) {
       const int i = l % nr, k = l / nr;
       T* line = base + (long long)k * nc * nr + i;
-      if (o.nyl > 0 && (o.byl == 1 || o.byl == 3)) bc3_side(line, nr, 1, o.nyl, o.byl, o.nyl + 1, 2 * o.nyl + 1, o.byl == 3 && m == 2);
-      if (o.jbeg > 0 && (o.byr == 1 || o.byr == 3)) bc3_side(line, nr, o.jbeg, nc, o.byr, o.jbeg - 1, 2 * o.jbeg - 1, o.byr == 3 && m == 2);
+      if (o.nyl > 0 && (o.byl == 1 || o.byl == 3)) bc3_side(line, nr, nc, 1, o.nyl, o.byl, o.nyl + 1, 2 * o.nyl + 1, o.byl == 3 && m == 2);
+      if (o.jbeg > 0 && (o.byr == 1 || o.byr == 3)) bc3_side(line, nr, nc, o.jbeg, nc, o.byr, o.jbeg - 1, 2 * o.jbeg - 1, o.byr == 3 && m == 2);
     } else {
       T* line = base + l;  // column (i,j) = (l % nr + 1, l / nr + 1)
       const long long st = (long long)nr * nc;
-      if (o.nzl > 0 && (o.bzl == 1 || o.bzl == 3)) bc3_side(line, st, 1, o.nzl, o.bzl, o.nzl + 1, 2 * o.nzl + 1, o.bzl == 3 && m == 3);
-      if (o.kbeg > 0 && (o.bzr == 1 || o.bzr == 3)) bc3_side(line, st, o.kbeg, nf, o.bzr, o.kbeg - 1, 2 * o.kbeg - 1, o.bzr == 3 && m == 3);
+      if (o.nzl > 0 && (o.bzl == 1 || o.bzl == 3)) bc3_side(line, st, nf, 1, o.nzl, o.bzl, o.nzl + 1, 2 * o.nzl + 1, o.bzl == 3 && m == 3);
+      if (o.kbeg > 0 && (o.bzr == 1 || o.bzr == 3)) bc3_side(line, st, nf, o.kbeg, nf, o.bzr, o.kbeg - 1, 2 * o.kbeg - 1, o.bzr == 3 && m == 3);
     }
   }
 }
