@@ -96,6 +96,7 @@ template <class T>
 struct Euler3Phys {
   static constexpr int NV = 5, NW = 3;
   Roe3T<T> R;
+  SplitRecip<T> rc;
   template <int DIR>
   __device__ __forceinline__ void load(const T*, const PatchDev&, long long, long long, long long, int) {}
   template <int DIR>
@@ -104,11 +105,16 @@ struct Euler3Phys {
   __device__ __forceinline__ void rpn(const Step3Params& sp, const T* QL, const T* QR, T (&W)[NW][NV], T* S, T* AM, T* AP) {
     R = roe3d((T)sp.gamma1, QL, QR);
     euler3d_rpn_roe((T)sp.gamma, (T)sp.gamma1, sp.efix != 0, DIR, QL, QR, R, W, S, AM, AP);
+    rc = split_recip(R.a);
   }
+  // FAST: the splits of euler3d_split_sub, for interfaces that quick() accepts
+  static constexpr bool HAS_QUICK = true;
   template <int DIR>
-  __device__ __forceinline__ void rpt(int, int icoor, const T* in, T* m, T* p) const { euler3d_trans(R, DIR, icoor, in, m, p); }
-  template <int DIR>
-  __device__ __forceinline__ void rptt(int, int icoor, int, const T* in, T* m, T* p) const { euler3d_trans(R, DIR, icoor, in, m, p); }
+  __device__ __forceinline__ bool quick() const { return euler3d_trans_sub(R, DIR); }
+  template <int DIR, bool FAST = false>
+  __device__ __forceinline__ void rpt(int, int icoor, const T* in, T* m, T* p) const { euler3d_trans<FAST>(R, rc, DIR, icoor, in, m, p); }
+  template <int DIR, bool FAST = false>
+  __device__ __forceinline__ void rptt(int, int icoor, int, const T* in, T* m, T* p) const { euler3d_trans<FAST>(R, rc, DIR, icoor, in, m, p); }
 };
 
 // Advection in a face-centred velocity field (aux 1..3 = u, v, w at the left x-, y- and
@@ -120,6 +126,9 @@ struct Euler3Phys {
 template <class T>
 struct Swirl3Phys {
   static constexpr int NV = 1, NW = 1;
+  static constexpr bool HAS_QUICK = false;
+  template <int DIR>
+  __device__ __forceinline__ bool quick() const { return false; }
   T un;
   // [0]: cell e-1, [1]: cell e. vy: y-like face velocity at (dy, dz) = (0,0), (+1,0),
   // (0,-1), (+1,-1), (0,+1), (+1,+1); vz: z-like one at (0,0), (0,+1), (-1,0), (-1,+1),
@@ -154,13 +163,13 @@ struct Swirl3Phys {
     AM[0] = dmin(un, T(0)) * W[0][0];
     AP[0] = dmax(un, T(0)) * W[0][0];
   }
-  template <int DIR>
+  template <int DIR, bool = false>
   __device__ __forceinline__ void rpt(int imp, int icoor, const T* in, T* m, T* p) const {
     const int c = imp - 1;
     if (icoor == 2) { m[0] = dmin(vy[c][0], T(0)) * in[0]; p[0] = dmax(vy[c][1], T(0)) * in[0]; }
     else { m[0] = dmin(vz[c][0], T(0)) * in[0]; p[0] = dmax(vz[c][1], T(0)) * in[0]; }
   }
-  template <int DIR>
+  template <int DIR, bool = false>
   __device__ __forceinline__ void rptt(int imp, int icoor, int impt, const T* in, T* m, T* p) const {
     const int c = imp - 1, o = impt == 1 ? 2 : 4;
     if (icoor == 2) { m[0] = dmin(vy[c][o], T(0)) * in[0]; p[0] = dmax(vy[c][o + 1], T(0)) * in[0]; }
@@ -183,7 +192,7 @@ static_assert(amrgpu_plugin::Check3D<Euler3Phys<float>, Step3Params, float>::val
 // made in an order that keeps few of them live at once: the z-like ones first (their
 // doubly transverse parts feed gadd), then the y-like ones; the hadd terms wait in shared
 // memory between their first summand and the rest.
-template <int DIR, class T, class PH>
+template <int DIR, bool FAST, class T, class PH>
 __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, const T* CQ, int m3, int m4, T dtdx, T dtdy,
                                            T dtdz, T* g) {
   constexpr int NV = PH::NV;
@@ -193,8 +202,8 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
   const bool first = imp == 2;
   // z-like split of the fluctuation and of the second-order part
   T cm[NV], cp[NV], cmq[NV], cpq[NV];
-  ph.template rpt<DIR>(imp, 3, F, cm, cp);
-  if (m3 == 2) ph.template rpt<DIR>(imp, 3, CQ, cmq, cpq);
+  ph.template rpt<DIR, FAST>(imp, 3, F, cm, cp);
+  if (m3 == 2) ph.template rpt<DIR, FAST>(imp, 3, CQ, cmq, cpq);
   else {
 #pragma unroll
     for (int m = 0; m < NV; ++m) cmq[m] = cpq[m] = T(0);
@@ -212,12 +221,12 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
     if (m4 > 0) {
       T t[NV];
       dt_input<NV>(m4, sgn3, cp, cpq, t);
-      ph.template rptt<DIR>(imp, 2, 2, t, P1, P2);
+      ph.template rptt<DIR, FAST>(imp, 2, 2, t, P1, P2);
       dt_input<NV>(m4, sgn3, cm, cmq, t);
-      ph.template rptt<DIR>(imp, 2, 1, t, M1, M2);
+      ph.template rptt<DIR, FAST>(imp, 2, 1, t, M1, M2);
     }
     T bm[NV], bp[NV];
-    ph.template rpt<DIR>(imp, 2, F, bm, bp);
+    ph.template rpt<DIR, FAST>(imp, 2, F, bm, bp);
 #pragma unroll
     for (int m = 0; m < NV; ++m) {
       T g01 = (first ? T(0) : G(1 * NV + m)) - T(0.5) * dtdx * bm[m];
@@ -246,7 +255,7 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
     }
     T bmq[NV], bpq[NV];
     if (m3 == 2) {
-      ph.template rpt<DIR>(imp, 2, CQ, bmq, bpq);
+      ph.template rpt<DIR, FAST>(imp, 2, CQ, bmq, bpq);
 #pragma unroll
       for (int m = 0; m < NV; ++m) {
         G(4 * NV + m) = first ? G(4 * NV + m) + dtdx * bpq[m] : G(4 * NV + m) - dtdx * bpq[m];
@@ -261,9 +270,9 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
     if (m4 > 0) {
       T t[NV];
       dt_input<NV>(m4, sgn3, bp, bpq, t);
-      ph.template rptt<DIR>(imp, 3, 2, t, X1, X2);
+      ph.template rptt<DIR, FAST>(imp, 3, 2, t, X1, X2);
       dt_input<NV>(m4, sgn3, bm, bmq, t);
-      ph.template rptt<DIR>(imp, 3, 1, t, Y1, Y2);
+      ph.template rptt<DIR, FAST>(imp, 3, 1, t, Y1, Y2);
     }
 #pragma unroll
     for (int m = 0; m < NV; ++m) {
@@ -353,7 +362,10 @@ __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, 
 #pragma unroll
       for (int m = 0; m < NV; ++m) sW[k * NV + m][l] = W[k][m];
   }
-  __syncthreads();
+  // (a plugin with a quick form of its splits takes it where every interface of the tile may)
+  bool quick = false;
+  if constexpr (PH::HAS_QUICK) quick = __syncthreads_and(!valid || ph.template quick<DIR>());
+  else __syncthreads();
   // interfaces 1..n1+1 carry fluxes; the tile edges only serve their neighbours
   const bool live = valid && e >= 1 && e <= n1 + 1 && l >= 1 && l <= SW_T - 2;
   const bool owned = live && l <= SW_T - 3;
@@ -410,11 +422,18 @@ __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, 
     }
   }
   __syncthreads();  // the waves in sW are read: the buffer takes the transverse terms now
-  // apdq side of interface e: the terms of cell e (flux3.f:429-505, 552-628 with i = e)
-  if (owned && e <= n1 && m3 > 0) trans_side<DIR, T, PH>(ph, 2, AP, CQ, m3, m4, dtdx, dtdy, dtdz, sG + l);
-  __syncthreads();
-  // amdq side of interface e: the terms of cell e-1, owned by thread l-1 of this tile
-  if (live && m3 > 0 && e >= 2 && l >= 2) trans_side<DIR, T, PH>(ph, 1, AM, CQ, m3, m4, dtdx, dtdy, dtdz, sG + (l - 1));
+  // apdq side of interface e: the terms of cell e (flux3.f:429-505, 552-628 with i = e), then
+  // the amdq side of interface e: the terms of cell e-1, owned by thread l-1 of this tile
+  auto transverse = [&](auto fast) {
+    constexpr bool F = decltype(fast)::value;
+    if (owned && e <= n1 && m3 > 0) trans_side<DIR, F, T, PH>(ph, 2, AP, CQ, m3, m4, dtdx, dtdy, dtdz, sG + l);
+    __syncthreads();
+    if (live && m3 > 0 && e >= 2 && l >= 2) trans_side<DIR, F, T, PH>(ph, 1, AM, CQ, m3, m4, dtdx, dtdy, dtdz, sG + (l - 1));
+  };
+  if constexpr (PH::HAS_QUICK) {
+    if (quick) transverse(std::true_type{});
+    else transverse(std::false_type{});
+  } else transverse(std::false_type{});
   __syncthreads();
   // the cell's transverse terms to the stash
   if (owned && e <= n1 && m3 > 0)
