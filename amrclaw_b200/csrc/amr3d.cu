@@ -1030,14 +1030,14 @@ class Amr3Gpu : public AmrSolver {
         const long long pencils = d == 0 ? (my + 2) * (mz + 2) : d == 1 ? (mx + 2) * (mz + 2) : (mx + 2) * (my + 2);
         L.sweep0[(size_t)d * (np + 1) + k] = slot;
         L.comp0[(size_t)d * (np + 1) + k] = comp;
-        slot += pencils * (n1 + 1);
+        slot += pencils * pencil_slots(n1);
         comp += pencils * (n1 + 3);
       }
       L.sweep0[(size_t)d * (np + 1) + np] = slot;
       L.comp0[(size_t)d * (np + 1) + np] = comp;
       L.items[d] = comp;
     }
-    L.slots = slot;
+    L.slots = stash_slots(slot);
     for (int k = 0; k < np; ++k) {
       const HPatch3& g = node[L.plist[k]];
       L.face0[k + 1] = L.face0[k] + (long long)(g.nx() + 1) * (g.ny() + 1) * (g.nz() + 1);
@@ -1524,7 +1524,7 @@ class Amr3Gpu : public AmrSolver {
     const double c = vel_period > 0.0 ? b4step_factor(t) : 1.0;
     Step3Args a{};
     a.pool = pool.d; a.patches = d_patches.d; a.sp = sp;
-    a.stash = d_stash.d; a.stash_stride = L.slots; a.flux = d_flux.d; a.flux_stride = L.faces;
+    a.stash = d_stash.d; a.flux = d_flux.d; a.flux_stride = L.faces;
     a.dt = dt; a.dt_dev = dtd; a.dx = hxposs[lev]; a.dy = hyposs[lev]; a.dz = hzposs[lev]; a.cflmax = d_cfl;
     AMR_CUDA(cudaMemsetAsync(d_cfl, 0, sizeof(unsigned long long), st));
     const double hx = hxposs[lev], hy = hyposs[lev], hz = hzposs[lev];
@@ -1814,7 +1814,7 @@ class Amr3Gpu : public AmrSolver {
           const long long n1 = d == 0 ? mx : d == 1 ? my : mz;
           const long long pencils = d == 0 ? (my + 2) * (mz + 2) : d == 1 ? (mx + 2) * (mz + 2) : (mx + 2) * (my + 2);
           sw[(size_t)d * (n + 1) + k] = slot; cp[(size_t)d * (n + 1) + k] = comp;
-          slot += pencils * (n1 + 1);
+          slot += pencils * pencil_slots(n1);
           comp += pencils * (n1 + 3);
         }
         sw[(size_t)d * (n + 1) + n] = slot; cp[(size_t)d * (n + 1) + n] = comp;
@@ -1826,7 +1826,7 @@ class Amr3Gpu : public AmrSolver {
         fc[k + 1] = fc[k] + (mx + 1) * (my + 1) * (mz + 1);
         ce[k + 1] = ce[k] + mx * my * mz;
       }
-      slots[li] = slot; faces[li] = fc[n]; cells[li] = ce[n];
+      slots[li] = stash_slots(slot); faces[li] = fc[n]; cells[li] = ce[n];
       pre.insert(pre.end(), sw.begin(), sw.end());
       pre.insert(pre.end(), cp.begin(), cp.end());
       pre.insert(pre.end(), fc.begin(), fc.end());
@@ -1852,7 +1852,7 @@ class Amr3Gpu : public AmrSolver {
       a.plist = rich_plist.d + li * np; a.np = np;
       const long long* b = rich_pre.d + base[li];
       a.sweep0 = b; a.comp0 = b + 3 * (np + 1); a.face0 = b + 6 * (np + 1); a.cell0 = b + 7 * (np + 1);
-      a.stash = d_stash.d; a.stash_stride = slots[li]; a.flux = d_flux.d; a.flux_stride = faces[li];
+      a.stash = d_stash.d; a.flux = d_flux.d; a.flux_stride = faces[li];
       a.dt = li == 0 ? 2.0 * dt : dt;
       a.dx = li == 0 ? 2.0 * hx : hx; a.dy = li == 0 ? 2.0 * hy : hy; a.dz = li == 0 ? 2.0 * hz : hz;
       a.cflmax = rich_cfl.d; a.queue = nullptr; a.dt_dev = nullptr;
@@ -2356,7 +2356,7 @@ class Amr3Gpu : public AmrSolver {
     {
       // sweep staging and face fluxes: reserved at once for twice a level-1 sweep
       const long long n = (long long)nxc * nyc * nzc;
-      d_stash.reserve((size_t)(stash_values(nvar) * 3 * (n + 4LL * (nxc * nyc + nyc * nzc + nxc * nzc))));
+      d_stash.reserve((size_t)(stash_values(nvar) * 3 * (n + 11LL * (nxc * nyc + nyc * nzc + nxc * nzc))));
       d_flux.reserve((size_t)(6 * nvar * (n + 2LL * (nxc * nyc + nyc * nzc + nxc * nzc) + 8)));
       d_stash.n = d_flux.n = 0;
     }

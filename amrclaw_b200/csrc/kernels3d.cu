@@ -80,11 +80,12 @@ constexpr int SW_OWN = SW_T - 3;
 template <class T>
 constexpr int sweep_min_blocks() { return sizeof(T) == 4 ? SW_MINB_F32 : SW_MINB; }
 
-// (a - 3*b) (m4 = 2) or a: the doubly transverse inputs of flux3.f:429-507
+// a -+ 3*b (m4 = 2) or a (w3 = 0: b's product is then a zero): the doubly transverse
+// inputs of flux3.f:429-507
 template <int NV, class T>
-__device__ __forceinline__ void dt_input(int m4, T sgn3, const T* a, const T* b, T* o) {
+__device__ __forceinline__ void dt_input(T w3, const T* a, const T* b, T* o) {
 #pragma unroll
-  for (int m = 0; m < NV; ++m) o[m] = (m4 == 2) ? a[m] + sgn3 * b[m] : a[m];
+  for (int m = 0; m < NV; ++m) o[m] = a[m] + w3 * b[m];
 }
 
 // ---- physics policies of the sweep: the problem's rpn3 / rpt3 / rptt3 at one interface.
@@ -198,8 +199,9 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
   constexpr int NV = PH::NV;
   auto G = [&](int x) -> T& { return g[x * SW_T]; };
   const T c6 = (T)(1.0 / 6.0);
-  const T sgn3 = imp == 2 ? T(-3) : T(3);
+  const T w3 = m4 == 2 ? (imp == 2 ? T(-3) : T(3)) : T(0);
   const bool first = imp == 2;
+  const T sdt = first ? dtdx : -dtdx;  // the second-order parts enter with opposite signs
   // z-like split of the fluctuation and of the second-order part
   T cm[NV], cp[NV], cmq[NV], cpq[NV];
   ph.template rpt<DIR, FAST>(imp, 3, F, cm, cp);
@@ -220,9 +222,9 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
     T P1[NV], P2[NV], M1[NV], M2[NV];
     if (m4 > 0) {
       T t[NV];
-      dt_input<NV>(m4, sgn3, cp, cpq, t);
+      dt_input<NV>(w3, cp, cpq, t);
       ph.template rptt<DIR, FAST>(imp, 2, 2, t, P1, P2);
-      dt_input<NV>(m4, sgn3, cm, cmq, t);
+      dt_input<NV>(w3, cm, cmq, t);
       ph.template rptt<DIR, FAST>(imp, 2, 1, t, M1, M2);
     }
     T bm[NV], bp[NV];
@@ -258,8 +260,8 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
       ph.template rpt<DIR, FAST>(imp, 2, CQ, bmq, bpq);
 #pragma unroll
       for (int m = 0; m < NV; ++m) {
-        G(4 * NV + m) = first ? G(4 * NV + m) + dtdx * bpq[m] : G(4 * NV + m) - dtdx * bpq[m];
-        G(1 * NV + m) = first ? G(1 * NV + m) + dtdx * bmq[m] : G(1 * NV + m) - dtdx * bmq[m];
+        G(4 * NV + m) = G(4 * NV + m) + sdt * bpq[m];
+        G(1 * NV + m) = G(1 * NV + m) + sdt * bmq[m];
       }
     } else {
 #pragma unroll
@@ -269,9 +271,9 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
     T X1[NV], X2[NV], Y1[NV], Y2[NV];
     if (m4 > 0) {
       T t[NV];
-      dt_input<NV>(m4, sgn3, bp, bpq, t);
+      dt_input<NV>(w3, bp, bpq, t);
       ph.template rptt<DIR, FAST>(imp, 3, 2, t, X1, X2);
-      dt_input<NV>(m4, sgn3, bm, bmq, t);
+      dt_input<NV>(w3, bm, bmq, t);
       ph.template rptt<DIR, FAST>(imp, 3, 1, t, Y1, Y2);
     }
 #pragma unroll
@@ -297,8 +299,8 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
         G(11 * NV + m) = T(0);
       }
       if (m3 == 2) {
-        h11 = first ? h11 + dtdx * cpq[m] : h11 - dtdx * cpq[m];
-        h01 = first ? h01 + dtdx * cmq[m] : h01 - dtdx * cmq[m];
+        h11 = h11 + sdt * cpq[m];
+        h01 = h01 + sdt * cmq[m];
       }
       G(7 * NV + m) = h01;
       G(10 * NV + m) = h11;
@@ -338,11 +340,11 @@ __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, 
     const int mx = P.ihi - P.ilo + 1, my = P.jhi - P.jlo + 1, mz = P.khi - P.klo + 1;
     n1 = DIR == 1 ? mx : DIR == 2 ? my : mz;
     const int n2 = DIR == 1 ? my : mx;
-    const long long loc = g - c0[pi];
-    e = (int)(loc % (n1 + 3));
-    const long long pen = loc / (n1 + 3);
-    const int a = (int)(pen % (n2 + 2)), b = (int)(pen / (n2 + 2));
-    slot = s0[pi] + pen * (n1 + 1) + (e - 1);
+    // (a patch's interfaces fit 32 bits: its stash alone would fill the device first)
+    const unsigned loc = (unsigned)(g - c0[pi]), pen = loc / (unsigned)(n1 + 3);
+    e = (int)(loc - pen * (unsigned)(n1 + 3));
+    const int b = (int)(pen / (unsigned)(n2 + 2)), a = (int)(pen - (unsigned)b * (unsigned)(n2 + 2));
+    slot = s0[pi] + pen * pencil_slots(n1) + (e - 1);
     const long long mi = P.mitot, mj = P.mjtot;
     long long base, step;  // enlarged-array index of pencil cell x is base + x*step (cell 0: enlarged index 1)
     if (DIR == 1) { base = ((long long)(b - 1 + NG3) * mj + (a - 1 + NG3)) * mi + (NG3 - 1); step = 1; }
@@ -373,8 +375,8 @@ __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, 
   T CQ[NV];
 #pragma unroll
   for (int m = 0; m < NV; ++m) CQ[m] = T(0);
-  T* st = static_cast<T*>(A.stash) + slot;
-  const long long ss = A.stash_stride;
+  T* st = static_cast<T*>(A.stash) + stash_at<NV>(slot);
+  constexpr int ss = STASH_BLK;
   const T c6 = (T)(1.0 / 6.0);
   const int m3 = sp.m3, m4 = sp.m4, order = sp.order;
   if (live) {
@@ -414,11 +416,11 @@ __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, 
       for (int m = 0; m < NV; ++m) {
         T fm = T(0) + AM[m], fp = T(0) - AP[m];
         if (order != 1) { fm = fm + CQ[m]; fp = fp + CQ[m]; }
-        st[(long long)m * ss] = fm;
-        st[(long long)(NV + m) * ss] = fp;
+        st[m * ss] = fm;
+        st[(NV + m) * ss] = fp;
       }
       if (e <= n1 && m3 <= 0)
-        for (int x = 2 * NV; x < stash_values(NV); ++x) st[(long long)x * ss] = T(0);
+        for (int x = 2 * NV; x < stash_values(NV); ++x) st[x * ss] = T(0);
     }
   }
   __syncthreads();  // the waves in sW are read: the buffer takes the transverse terms now
@@ -437,7 +439,7 @@ __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, 
   __syncthreads();
   // the cell's transverse terms to the stash
   if (owned && e <= n1 && m3 > 0)
-    for (int x = 0; x < 12 * NV; ++x) st[(long long)(2 * NV + x) * ss] = G(x, l);
+    for (int x = 0; x < 12 * NV; ++x) st[(2 * NV + x) * ss] = G(x, l);
   // block-wide max of the Courant number, one atomic per warp
   for (int o = 16; o > 0; o >>= 1) cfl = dmax(cfl, __shfl_xor_sync(0xffffffffu, cfl, o));
   if ((threadIdx.x & 31) == 0 && cfl > T(0)) atomic_max_nonneg(A.cflmax, (double)cfl);
@@ -631,12 +633,12 @@ template <int NV>
 __device__ __forceinline__ int hidx(int s, int d, int m) { return 8 * NV + ((s - 1) * 3 + (d + 1)) * NV + m; }
 
 // ------------------------------------------------------------------- faces
-constexpr int FB_I = 8, FB_J = 4, FB_K = 4;  // face bricks: one warp per k-plane, a block per brick
+constexpr int FB_I = 4, FB_J = 4, FB_K = 8;  // face bricks: four warps of 4 x 4 x 2 faces
 template <class T, int NV>
 __global__ void __launch_bounds__(128) face3_kernel(Step3Args A) {
   // face cells [face0[0], face0[np]): the level's, or one patch's through a one-patch view
   const long long first = A.face0[0], total = A.face0[A.np];
-  const long long ss = A.stash_stride;
+  constexpr int ss = STASH_BLK;
   const T* S = static_cast<const T*>(A.stash);
   for (long long t = first + (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     const int pi = find_patch(A.face0, A.np, t);
@@ -644,31 +646,33 @@ __global__ void __launch_bounds__(128) face3_kernel(Step3Args A) {
     const int mx = P.ihi - P.ilo + 1, my = P.jhi - P.jlo + 1, mz = P.khi - P.klo + 1;
     // Thread t takes the face cells of its patch in brick order: slabs of FB_K k-planes,
     // rows of FB_J j-lines in a slab, bricks of FB_I faces in a row (the last of each
-    // smaller), i fastest inside a brick. A warp then reads the j- and k-contiguous
-    // stashes of the y and z sweeps in whole sectors, and the warps of a block share
-    // them through L1. The sums of every face are the same; only which thread makes
-    // them changes.
+    // smaller). Inside a whole brick a warp takes 4 x 4 x 2 faces, so that it reads four
+    // consecutive interfaces of every x and y pencil it touches, and the block the eight of
+    // a z pencil that share a 64-byte piece of DRAM: on a 90^3 level the kernel's DRAM reads
+    // fell from 1.73 to 1.40 GB (the stash is 1.32 GB) and its time from 376 to 330 us
+    // against 8 x 4 x 4 bricks over unaligned pencils. The sums of every face are the same;
+    // only which thread makes them changes.
     const int NI = mx + 1, NJ = my + 1, NK = mz + 1;
-    const long long loc = t - A.face0[pi];
-    const long long slab = (long long)NI * NJ * FB_K;
+    const unsigned loc = (unsigned)(t - A.face0[pi]);
+    const unsigned slab = (unsigned)(NI * NJ) * FB_K;
     const int kb = (int)(loc / slab);
     const int kcnt = min(FB_K, NK - kb * FB_K);
-    const long long r1 = loc - kb * slab;
-    const long long row = (long long)NI * FB_J * kcnt;
+    const unsigned r1 = loc - (unsigned)kb * slab;
+    const unsigned row = (unsigned)(NI * FB_J * kcnt);
     const int jb = (int)(r1 / row);
     const int jcnt = min(FB_J, NJ - jb * FB_J);
-    const int r2 = (int)(r1 - jb * row);
+    const int r2 = (int)(r1 - (unsigned)jb * row);
     const int bsz = FB_I * jcnt * kcnt;
     const int ib = r2 / bsz;
     const int icnt = min(FB_I, NI - ib * FB_I);
     const int r3 = r2 - ib * bsz;
-    const int i = ib * FB_I + r3 % icnt + 1;
-    const int j = jb * FB_J + (r3 / icnt) % jcnt + 1;
-    const int k = kb * FB_K + r3 / (icnt * jcnt) + 1;
+    const int i0 = r3 % icnt, j0 = (r3 / icnt) % jcnt, k0 = r3 / (icnt * jcnt);
+    const int i = ib * FB_I + i0 + 1, j = jb * FB_J + j0 + 1, k = kb * FB_K + k0 + 1;
     const long long bx = A.sweep0[pi], by = A.sweep0[(A.np + 1) + pi], bz = A.sweep0[2 * (A.np + 1) + pi];
-    auto xs = [&](int jj, int kk, int ii) { return bx + ((long long)(kk * (my + 2) + jj) * (mx + 1) + (ii - 1)); };
-    auto ys = [&](int ii, int kk, int jj) { return by + ((long long)(kk * (mx + 2) + ii) * (my + 1) + (jj - 1)); };
-    auto zs = [&](int ii, int jj, int kk) { return bz + ((long long)(jj * (mx + 2) + ii) * (mz + 1) + (kk - 1)); };
+    const int px = (int)pencil_slots(mx), py = (int)pencil_slots(my), pz = (int)pencil_slots(mz);
+    auto xs = [&](int jj, int kk, int ii) { return stash_at<NV>(bx + ((long long)(kk * (my + 2) + jj) * px + (ii - 1))); };
+    auto ys = [&](int ii, int kk, int jj) { return stash_at<NV>(by + ((long long)(kk * (mx + 2) + ii) * py + (jj - 1))); };
+    auto zs = [&](int ii, int jj, int kk) { return stash_at<NV>(bz + ((long long)(jj * (mx + 2) + ii) * pz + (kk - 1))); };
     T* F = static_cast<T*>(A.flux) + A.face0[pi] + ((long long)(k - 1) * NJ + (j - 1)) * NI + (i - 1);
     const long long fs = A.flux_stride;
     if (j <= my && k <= mz) {  // x-face i
