@@ -99,31 +99,44 @@ struct Acoustics2 {
 };
 
 // ---------------------------------------------------------------- euler (Roe)
+// Roe average of an interface: the normal and transverse velocities of the sweep (u, v),
+// enthalpy and sound speed, with the combinations the wave decompositions use.
+template <class R> struct Roe2 { R u, v, enth, u2v2, a, g1a2, euv; };
+
 struct Euler2 {
   static constexpr int MEQN = 4, MWAVES = 4, NAUX = 0;
   template <class R>
-  __device__ static void rpn(const ProbDev& P, int ixy, const R* qL, const R* qR, const R*, const R*,
-                             R (&wave)[MWAVES][MEQN], R (&s)[MWAVES], R (&amdq)[MEQN], R (&apdq)[MEQN]) {
-    const int mu = (ixy == 1) ? 1 : 2, mv = (ixy == 1) ? 2 : 1;
-    const R g1 = R(P.gamma1), gam = R(P.gamma);
+  __device__ __forceinline__ static Roe2<R> roe(R g1, int mu, int mv, const R* qL, const R* qR, R& pl, R& pr) {
     const R rl = qL[0], rr = qR[0];
     const R sql = sqrt(rl), sqr = sqrt(rr);
-    const R pl = g1 * (qL[3] - R(0.5) * (qL[mu] * qL[mu] + qL[mv] * qL[mv]) / rl);
-    const R pr = g1 * (qR[3] - R(0.5) * (qR[mu] * qR[mu] + qR[mv] * qR[mv]) / rr);
+    pl = g1 * (qL[3] - R(0.5) * (qL[mu] * qL[mu] + qL[mv] * qL[mv]) / rl);
+    pr = g1 * (qR[3] - R(0.5) * (qR[mu] * qR[mu] + qR[mv] * qR[mv]) / rr);
     const R rsum = sql + sqr;
-    const R u = (qL[mu] / sql + qR[mu] / sqr) / rsum;
-    const R v = (qL[mv] / sql + qR[mv] / sqr) / rsum;
-    const R enth = ((qL[3] + pl) / sql + (qR[3] + pr) / sqr) / rsum;
-    const R u2v2 = u * u + v * v;
-    const R a2 = g1 * (enth - R(0.5) * u2v2);
-    const R a = sqrt(a2);
-    const R g1a2 = g1 / a2;
-    const R euv = enth - u2v2;
+    Roe2<R> o;
+    o.u = (qL[mu] / sql + qR[mu] / sqr) / rsum;
+    o.v = (qL[mv] / sql + qR[mv] / sqr) / rsum;
+    o.enth = ((qL[3] + pl) / sql + (qR[3] + pr) / sqr) / rsum;
+    o.u2v2 = o.u * o.u + o.v * o.v;
+    const R a2 = g1 * (o.enth - R(0.5) * o.u2v2);
+    o.a = sqrt(a2);
+    o.g1a2 = g1 / a2;
+    o.euv = o.enth - o.u2v2;
+    return o;
+  }
+  // rpn2 with the interface's Roe average handed on for its transverse splits
+  template <class R>
+  __device__ __forceinline__ static void rpn_roe(const ProbDev& P, int ixy, const R* qL, const R* qR, Roe2<R>& o,
+                                                 R (&wave)[MWAVES][MEQN], R (&s)[MWAVES], R (&amdq)[MEQN], R (&apdq)[MEQN]) {
+    const int mu = (ixy == 1) ? 1 : 2, mv = (ixy == 1) ? 2 : 1;
+    const R g1 = R(P.gamma1), gam = R(P.gamma);
+    R pl, pr;
+    o = roe<R>(g1, mu, mv, qL, qR, pl, pr);
+    const R u = o.u, v = o.v, a = o.a, enth = o.enth, u2v2 = o.u2v2;
     const R d1 = qR[0] - qL[0];
     const R d2 = qR[mu] - qL[mu];
     const R d3 = qR[mv] - qL[mv];
     const R d4 = qR[3] - qL[3];
-    const R ae = g1a2 * (euv * d1 + u * d2 + v * d3 - d4);
+    const R ae = o.g1a2 * (o.euv * d1 + u * d2 + v * d3 - d4);
     const R as = d3 - v * d1;
     const R a4 = (d2 + (a - u) * d1 - a * ae) / (R(2) * a);
     const R a1 = d1 - ae - a4;
@@ -139,29 +152,32 @@ struct Euler2 {
       for (int mw = 0; mw < 4; ++mw) t = t + s[mw] * wave[mw][m];
       df[m] = t;
     }
+    // the entropy fix looks at a sonic point only where the wave speed's sign allows one
     bool fixed = false;
     if (P.efix) {
-      const R cl = sqrt(gam * pl / rl);
-      const R sl = qL[mu] / rl - cl;
-      if (sl < R(0) && s[0] > R(0)) {
-        const R r1 = qL[0] + wave[0][0];
-        const R ru1 = qL[mu] + wave[0][mu];
-        const R rv1 = qL[mv] + wave[0][mv];
-        const R e1 = qL[3] + wave[0][3];
-        const R p1 = g1 * (e1 - R(0.5) * (ru1 * ru1 + rv1 * rv1) / r1);
-        const R c1 = sqrt(gam * p1 / r1);
-        const R sr = ru1 / r1 - c1;
-        if (sr > R(0)) {
-          const R sfract = sl * (sr - s[0]) / (sr - sl);
+      if (s[0] > R(0)) {
+        const R cl = sqrt(gam * pl / qL[0]);
+        const R sl = qL[mu] / qL[0] - cl;
+        if (sl < R(0)) {
+          const R r1 = qL[0] + wave[0][0];
+          const R ru1 = qL[mu] + wave[0][mu];
+          const R rv1 = qL[mv] + wave[0][mv];
+          const R e1 = qL[3] + wave[0][3];
+          const R p1 = g1 * (e1 - R(0.5) * (ru1 * ru1 + rv1 * rv1) / r1);
+          const R c1 = sqrt(gam * p1 / r1);
+          const R sr = ru1 / r1 - c1;
+          if (sr > R(0)) {
+            const R sfract = sl * (sr - s[0]) / (sr - sl);
 #pragma unroll
-          for (int m = 0; m < 4; ++m) { amdq[m] = sfract * wave[0][m]; apdq[m] = df[m] - amdq[m]; }
-          fixed = true;
+            for (int m = 0; m < 4; ++m) { amdq[m] = sfract * wave[0][m]; apdq[m] = df[m] - amdq[m]; }
+            fixed = true;
+          }
         }
       }
-      if (!fixed) {
-        const R cr = sqrt(gam * pr / rr);
-        const R sr = qR[mu] / rr + cr;
-        if (s[3] < R(0) && sr > R(0)) {
+      if (!fixed && s[3] < R(0)) {
+        const R cr = sqrt(gam * pr / qR[0]);
+        const R sr = qR[mu] / qR[0] + cr;
+        if (sr > R(0)) {
           const R r3 = qR[0] - wave[3][0];
           const R ru3 = qR[mu] - wave[3][mu];
           const R rv3 = qR[mv] - wave[3][mv];
@@ -190,29 +206,47 @@ struct Euler2 {
       }
     }
   }
+  // rpt2 from the Roe average of the interface
   template <class R>
-  __device__ static void rpt(const ProbDev& P, int ixy, int imp, const R* qL, const R* qR, const R*, const R*,
-                             const R*, const R* asdq, R (&bm)[MEQN], R (&bp)[MEQN]) {
+  __device__ __forceinline__ static void rpt_roe(const Roe2<R>& o, int ixy, const R* asdq, R (&bm)[MEQN], R (&bp)[MEQN]) {
     const int mu = (ixy == 1) ? 1 : 2, mv = (ixy == 1) ? 2 : 1;
-    const R g1 = R(P.gamma1);
-    const R rl = qL[0], rr = qR[0];
-    const R sql = sqrt(rl), sqr = sqrt(rr);
-    const R pl = g1 * (qL[3] - R(0.5) * (qL[mu] * qL[mu] + qL[mv] * qL[mv]) / rl);
-    const R pr = g1 * (qR[3] - R(0.5) * (qR[mu] * qR[mu] + qR[mv] * qR[mv]) / rr);
-    const R rsum = sql + sqr;
-    const R u = (qL[mu] / sql + qR[mu] / sqr) / rsum;
-    const R v = (qL[mv] / sql + qR[mv] / sqr) / rsum;
-    const R enth = ((qL[3] + pl) / sql + (qR[3] + pr) / sqr) / rsum;
-    const R u2v2 = u * u + v * v;
-    const R a2 = g1 * (enth - R(0.5) * u2v2);
-    const R a = sqrt(a2);
-    const R g1a2 = g1 / a2;
-    const R euv = enth - u2v2;
+    const R u = o.u, v = o.v, a = o.a, enth = o.enth, u2v2 = o.u2v2;
     const R d1 = asdq[0], dmu = asdq[mu], dmv = asdq[mv], d4 = asdq[3];
-    const R ae = g1a2 * (euv * d1 + u * dmu + v * dmv - d4);
+    const R ae = o.g1a2 * (o.euv * d1 + u * dmu + v * dmv - d4);
     const R as = dmu - u * d1;
     const R a4 = (dmv + (a - v) * d1 - a * ae) / (R(2) * a);
     const R a1 = d1 - ae - a4;
+    // the waves' terms s_k w_k go to the minus or the plus side by the sign of s_k; the other
+    // side's term is a zero, and leaving a zero out of a sum that starts from +0 changes no
+    // value. (A wave that is not finite would make that zero a NaN: the general form below.)
+    const R s0 = v - a, s3 = v + a;
+    const bool finite = isfinite(a4);
+    if (finite && s0 < R(0) && s3 > R(0)) {
+      const R m = dmin(v, R(0)), p = dmax(v, R(0));
+      R w1 = ae;
+      bm[0] = s0 * a1 + m * w1; bp[0] = p * w1 + s3 * a4;
+      w1 = ae * u;
+      R w2 = as;
+      bm[mu] = s0 * (a1 * u) + m * w1 + m * w2; bp[mu] = p * w1 + p * w2 + s3 * (a4 * u);
+      w1 = ae * v;
+      bm[mv] = s0 * (a1 * s0) + m * w1; bp[mv] = p * w1 + s3 * (a4 * s3);
+      w1 = ae * R(0.5) * u2v2;
+      w2 = as * u;
+      bm[3] = s0 * (a1 * (enth - v * a)) + m * w1 + m * w2; bp[3] = p * w1 + p * w2 + s3 * (a4 * (enth + v * a));
+      return;
+    }
+    if (finite && (s0 > R(0) || s3 < R(0))) {
+      // all waves move to one side
+      R t[4];
+      t[0] = s0 * a1 + v * ae + s3 * a4;
+      t[mu] = s0 * (a1 * u) + v * (ae * u) + v * as + s3 * (a4 * u);
+      t[mv] = s0 * (a1 * s0) + v * (ae * v) + s3 * (a4 * s3);
+      t[3] = s0 * (a1 * (enth - v * a)) + v * (ae * R(0.5) * u2v2) + v * (as * u) + s3 * (a4 * (enth + v * a));
+      const bool plus = s0 > R(0);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) { bm[m] = plus ? R(0) : t[m]; bp[m] = plus ? t[m] : R(0); }
+      return;
+    }
     R w[4][4], sp[4];
     w[0][0] = a1; w[0][mu] = a1 * u; w[0][mv] = a1 * (v - a); w[0][3] = a1 * (enth - v * a); sp[0] = v - a;
     w[1][0] = ae; w[1][mu] = ae * u; w[1][mv] = ae * v; w[1][3] = ae * R(0.5) * u2v2; sp[1] = v;
@@ -228,6 +262,19 @@ struct Euler2 {
       }
       bm[m] = b_m; bp[m] = b_p;
     }
+  }
+  template <class R>
+  __device__ static void rpn(const ProbDev& P, int ixy, const R* qL, const R* qR, const R*, const R*,
+                             R (&wave)[MWAVES][MEQN], R (&s)[MWAVES], R (&amdq)[MEQN], R (&apdq)[MEQN]) {
+    Roe2<R> o;
+    rpn_roe<R>(P, ixy, qL, qR, o, wave, s, amdq, apdq);
+  }
+  template <class R>
+  __device__ static void rpt(const ProbDev& P, int ixy, int imp, const R* qL, const R* qR, const R*, const R*,
+                             const R*, const R* asdq, R (&bm)[MEQN], R (&bp)[MEQN]) {
+    const int mu = (ixy == 1) ? 1 : 2, mv = (ixy == 1) ? 2 : 1;
+    R pl, pr;
+    rpt_roe<R>(roe<R>(R(P.gamma1), mu, mv, qL, qR, pl, pr), ixy, asdq, bm, bp);
   }
 };
 
@@ -254,6 +301,36 @@ struct VcAdvection2 {
     const int kv = 3 - ixy;
     bm[0] = dmin(aux2[kv - 1], R(0)) * asdq[0];
     bp[0] = dmax(aux3[kv - 1], R(0)) * asdq[0];
+  }
+};
+
+// What an interface keeps between its rpn2 and its two rpt2 calls. A plugin's rpt2 is given
+// the states again; Euler's needs only their Roe average, which rpn2 has made.
+template <class S, class R>
+struct Iface2 {
+  __device__ __forceinline__ void rpn(const ProbDev& P, int ixy, const R* qL, const R* qR, const R* auxL, const R* auxR,
+                                      R (&wave)[S::MWAVES][S::MEQN], R (&s)[S::MWAVES], R (&amdq)[S::MEQN], R (&apdq)[S::MEQN]) {
+    S::template rpn<R>(P, ixy, qL, qR, auxL, auxR, wave, s, amdq, apdq);
+  }
+  template <class LoadQ>
+  __device__ __forceinline__ void rpt(const ProbDev& P, int ixy, int imp, LoadQ loadq, const R* aux1, const R* aux2,
+                                      const R* aux3, const R* asdq, R (&bm)[S::MEQN], R (&bp)[S::MEQN]) const {
+    R qL[S::MEQN], qR[S::MEQN];
+    loadq(qL, qR);
+    S::template rpt<R>(P, ixy, imp, qL, qR, aux1, aux2, aux3, asdq, bm, bp);
+  }
+};
+template <class R>
+struct Iface2<Euler2, R> {
+  Roe2<R> o;
+  __device__ __forceinline__ void rpn(const ProbDev& P, int ixy, const R* qL, const R* qR, const R*, const R*,
+                                      R (&wave)[4][4], R (&s)[4], R (&amdq)[4], R (&apdq)[4]) {
+    Euler2::rpn_roe<R>(P, ixy, qL, qR, o, wave, s, amdq, apdq);
+  }
+  template <class LoadQ>
+  __device__ __forceinline__ void rpt(const ProbDev&, int ixy, int, LoadQ, const R*, const R*, const R*, const R* asdq,
+                                      R (&bm)[4], R (&bp)[4]) const {
+    Euler2::rpt_roe<R>(o, ixy, asdq, bm, bp);
   }
 };
 
