@@ -105,87 +105,6 @@ struct AuxCell {
   }
 };
 
-// flux2.f:136-194 at one face from the wave records (waves, speeds, amdq, apdq) of the face
-// (rc) and of its neighbours (rm: face f-1, rp: face f+1): limiter.f's limited waves, the
-// second-order correction cqxx, fm = (0 + amdq) + cqxx/2 and fp = (0 - apdq) + cqxx/2
-// dl, dr: dtdx1d of the cells left and right of the face (dt/dx, divided by the capacity of
-// the cell when there is one: step2.f90:83-88)
-template <class S, class R>
-__device__ __forceinline__ void face_fluxes(const StepParams& sp, const R* rm, const R* rc, const R* rp, R dl, R dr,
-                                            R (&amdq)[S::MEQN], R (&apdq)[S::MEQN], R (&cqxx)[S::MEQN],
-                                            R (&fm)[S::MEQN], R (&fp)[S::MEQN]) {
-  constexpr int ME = S::MEQN, MW = S::MWAVES;
-#pragma unroll
-  for (int m = 0; m < ME; ++m) { amdq[m] = rc[MW * ME + MW + m]; apdq[m] = rc[MW * ME + MW + ME + m]; }
-#pragma unroll
-  for (int m = 0; m < ME; ++m) { fm[m] = R(0) + amdq[m]; fp[m] = R(0) - apdq[m]; cqxx[m] = R(0); }
-  if (sp.order == 1) return;
-  R wl[MW][ME];
-#pragma unroll
-  for (int mw = 0; mw < MW; ++mw) {
-    const R smw = rc[MW * ME + mw];
-#pragma unroll
-    for (int m = 0; m < ME; ++m) wl[mw][m] = rc[mw * ME + m];
-    if (sp.mthlim[mw] == 0) continue;
-    R wn2 = R(0), dotl = R(0), dotr = R(0);
-#pragma unroll
-    for (int m = 0; m < ME; ++m) {
-      wn2 = wn2 + rc[mw * ME + m] * rc[mw * ME + m];
-      dotl = dotl + rm[mw * ME + m] * rc[mw * ME + m];
-      dotr = dotr + rc[mw * ME + m] * rp[mw * ME + m];
-    }
-    if (wn2 == R(0)) continue;
-    const R r = (smw > R(0)) ? dotl / wn2 : dotr / wn2;
-    R wlim = R(0);
-    switch (sp.mthlim[mw]) {
-      case 1: wlim = dmax(R(0), dmin(R(1), r)); break;
-      case 2: wlim = dmax(R(0), dmax(dmin(R(1), R(2) * r), dmin(R(2), r))); break;
-      case 3: wlim = (r + fabs(r)) / (R(1) + fabs(r)); break;
-      case 4: { const R c = (R(1) + r) / R(2); wlim = dmax(R(0), dmin(c, dmin(R(2), R(2) * r))); } break;
-      case 5: wlim = r; break;
-    }
-#pragma unroll
-    for (int m = 0; m < ME; ++m) wl[mw][m] = wlim * wl[mw][m];
-  }
-  const R dtdxave = R(0.5) * (dl + dr);
-#pragma unroll
-  for (int m = 0; m < ME; ++m) {
-    R c = R(0);
-#pragma unroll
-    for (int mw = 0; mw < MW; ++mw) {
-      const R smw = rc[MW * ME + mw];
-      const R abs_sign = sp.use_fwaves ? dsign(R(1), smw) : fabs(smw);
-      c = c + abs_sign * (R(1) - fabs(smw) * dtdxave) * wl[mw][m];
-    }
-    cqxx[m] = c;
-    fm[m] = fm[m] + R(0.5) * c;
-    fp[m] = fp[m] + R(0.5) * c;
-  }
-}
-
-// rpn2 at one face into its wave record: waves [MW][ME], speeds [MW], amdq [ME], apdq [ME].
-// auxL, auxR: aux of the cells left and right of the face; dl, dr: their dtdx1d (flux2.f's
-// Courant number takes dtdx1d(i)*s and -dtdx1d(i-1)*s)
-template <class S, class R>
-__device__ __forceinline__ void face_record(const StepParams& sp, int ixy, const R* qL, const R* qR, const R* auxL,
-                                            const R* auxR, R* rec, R dl, R dr, bool count_cfl, R& cfl) {
-  constexpr int ME = S::MEQN, MW = S::MWAVES;
-  R wave[MW][ME], s[MW], amdq[ME], apdq[ME];
-  S::template rpn<R>(sp.prob, ixy, qL, qR, auxL, auxR, wave, s, amdq, apdq);
-#pragma unroll
-  for (int mw = 0; mw < MW; ++mw) {
-#pragma unroll
-    for (int m = 0; m < ME; ++m) rec[mw * ME + m] = wave[mw][m];
-    rec[MW * ME + mw] = s[mw];
-  }
-#pragma unroll
-  for (int m = 0; m < ME; ++m) { rec[MW * ME + MW + m] = amdq[m]; rec[MW * ME + MW + ME + m] = apdq[m]; }
-  if (count_cfl) {
-#pragma unroll
-    for (int mw = 0; mw < MW; ++mw) cfl = dmax(cfl, dmax(dr * s[mw], -dl * s[mw]));
-  }
-}
-
 // limiter.f's limiter function of the wave ratio r
 template <class R>
 __device__ __forceinline__ R philim2(int meth, R r) {
@@ -197,6 +116,45 @@ __device__ __forceinline__ R philim2(int meth, R r) {
     case 5: return r;
   }
   return R(0);
+}
+
+// flux2.f:136-194 at one face whose waves, and those of the faces before and after it along
+// the line (threads tid -+ nb), are in X: limited waves, the second-order correction cq,
+// fm = (0 + amdq) + cq/2 and fp = (0 - apdq) + cq/2. dl, dr: dtdx1d of the cells left and
+// right of the face (dt/dx, divided by the capacity of the cell when there is one:
+// step2.f90:83-88)
+template <class S, class R>
+__device__ __forceinline__ void limited_fluxes(const StepParams& sp, const R* X, int pitch, int tid, int nb, R dl, R dr,
+                                               const R (&s)[S::MWAVES], const R (&amdq)[S::MEQN], const R (&apdq)[S::MEQN],
+                                               R (&cq)[S::MEQN], R (&fm)[S::MEQN], R (&fp)[S::MEQN]) {
+  constexpr int ME = S::MEQN, MW = S::MWAVES;
+#pragma unroll
+  for (int m = 0; m < ME; ++m) { cq[m] = R(0); fm[m] = R(0) + amdq[m]; fp[m] = R(0) - apdq[m]; }
+  if (sp.order == 1) return;
+  const R dtdxave = R(0.5) * (dl + dr);
+#pragma unroll
+  for (int mw = 0; mw < MW; ++mw) {
+    R w[ME];
+#pragma unroll
+    for (int m = 0; m < ME; ++m) w[m] = X[(mw * ME + m) * pitch + tid];
+    if (sp.mthlim[mw] != 0) {
+      // the ratio takes the neighbour on the upwind side
+      const R* wn = X + mw * ME * pitch + tid + (s[mw] > R(0) ? -nb : nb);
+      R wn2 = R(0), dot = R(0);
+#pragma unroll
+      for (int m = 0; m < ME; ++m) { wn2 = wn2 + w[m] * w[m]; dot = dot + wn[m * pitch] * w[m]; }
+      if (wn2 != R(0)) {
+        const R phi = philim2(sp.mthlim[mw], dot / wn2);
+#pragma unroll
+        for (int m = 0; m < ME; ++m) w[m] = phi * w[m];
+      }
+    }
+    const R c = (sp.use_fwaves ? dsign(R(1), s[mw]) : fabs(s[mw])) * (R(1) - fabs(s[mw]) * dtdxave);
+#pragma unroll
+    for (int m = 0; m < ME; ++m) cq[m] = cq[m] + c * w[m];
+  }
+#pragma unroll
+  for (int m = 0; m < ME; ++m) { fm[m] = fm[m] + R(0.5) * cq[m]; fp[m] = fp[m] + R(0.5) * cq[m]; }
 }
 
 // One sweep direction of flux2.f over the tile. IXY = 1: lines are rows, IXY = 2: columns.
@@ -260,36 +218,8 @@ __device__ __forceinline__ void step2_sweep(const StepParams& sp, const R* Qs, c
   const bool split = flux && sp.trans != 0;
   R am2[ME], ap2[ME];
   if (flux) {
-    constexpr int NB = IXY == 1 ? 1 : L::NLINE;
     R cq[ME], fm[ME], fp[ME];
-#pragma unroll
-    for (int m = 0; m < ME; ++m) { cq[m] = R(0); fm[m] = R(0) + amdq[m]; fp[m] = R(0) - apdq[m]; }
-    if (sp.order != 1) {
-      const R dtdxave = R(0.5) * (dl + dr);
-#pragma unroll
-      for (int mw = 0; mw < MW; ++mw) {
-        R w[ME];
-#pragma unroll
-        for (int m = 0; m < ME; ++m) w[m] = X[(mw * ME + m) * PITCH + tid];
-        if (sp.mthlim[mw] != 0) {
-          // the ratio takes the neighbour on the upwind side
-          const R* wn = X + mw * ME * PITCH + tid + (s[mw] > R(0) ? -NB : NB);
-          R wn2 = R(0), dot = R(0);
-#pragma unroll
-          for (int m = 0; m < ME; ++m) { wn2 = wn2 + w[m] * w[m]; dot = dot + wn[m * PITCH] * w[m]; }
-          if (wn2 != R(0)) {
-            const R phi = philim2(sp.mthlim[mw], dot / wn2);
-#pragma unroll
-            for (int m = 0; m < ME; ++m) w[m] = phi * w[m];
-          }
-        }
-        const R c = (sp.use_fwaves ? dsign(R(1), s[mw]) : fabs(s[mw])) * (R(1) - fabs(s[mw]) * dtdxave);
-#pragma unroll
-        for (int m = 0; m < ME; ++m) cq[m] = cq[m] + c * w[m];
-      }
-#pragma unroll
-      for (int m = 0; m < ME; ++m) { fm[m] = fm[m] + R(0.5) * cq[m]; fp[m] = fp[m] + R(0.5) * cq[m]; }
-    }
+    limited_fluxes<S, R>(sp, X, PITCH, tid, IXY == 1 ? 1 : L::NLINE, dl, dr, s, amdq, apdq, cq, fm, fp);
     const int lin = line - 1, fa = ff - 1;
     if (lin >= 0 && lin < nt) {
 #pragma unroll
@@ -354,7 +284,7 @@ __device__ __forceinline__ void register_epilogue(const StepArgs& a, const StepW
                                                   const R* GP, int xrows) {
   constexpr int T = TILE2;
   const int tid = threadIdx.x;
-  for (int it = tid; it < wk.fsv_count * ME; it += STEP2_THREADS) {
+  for (int it = tid; it < wk.fsv_count * ME; it += blockDim.x) {
     const FsvEntry e = a.fsv[wk.fsv_start + it / ME];
     const int m = it % ME;
     const int ca = e.ic - i0, rb = e.jc - j0;
@@ -365,7 +295,7 @@ __device__ __forceinline__ void register_epilogue(const StepArgs& a, const StepW
     else v = -(double)GP[(m * (T + 1) + rb) * T + ca] * dt * a.dx;
     a.regs[e.dst + m] = v;
   }
-  for (int it = tid; it < wk.fad_count * ME; it += STEP2_THREADS) {
+  for (int it = tid; it < wk.fad_count * ME; it += blockDim.x) {
     const FadEntry e = a.fad[wk.fad_start + it / ME];
     const int m = it % ME;
     const int r = e.pad;
@@ -391,7 +321,7 @@ __device__ __forceinline__ void cfl_to_level(R cfl, R* red, unsigned long long* 
   __syncthreads();
   if (tid == 0) {
     R c = R(0);
-    for (int k = 0; k < STEP2_THREADS / 32; ++k) c = dmax(c, red[k]);
+    for (int k = 0; k < (int)blockDim.x / 32; ++k) c = dmax(c, red[k]);
     atomicMax(cflmax, (unsigned long long)__double_as_longlong((double)c));
   }
 }
@@ -618,24 +548,58 @@ __global__ void __launch_bounds__(STEP2_THREADS, step2_blocks<S, R>()) step2_bat
 // takes every face each tile computes (the maximum is unchanged by faces counted twice).
 // Face fluxes are fm = (0 + amdq) + cqxx/2, fp = (0 - apdq) + cqxx/2: flux2_dimSplit's
 // faddm = amdq, faddp = -apdq (+ cqxx/2) added to zeroed arrays give the same values.
+// As in the unsplit step a sweep is one round, a thread per face: 20 rows of 19 faces in x,
+// 16 columns of 19 in y.
 template <class S>
 struct Split2Layout {
-  static constexpr int ME = S::MEQN, MW = S::MWAVES, T = TILE2, QW = T + 4;
+  static constexpr int ME = S::MEQN, MW = S::MWAVES, T = TILE2, QW = T + 4, NFACE = T + 3;
+  static constexpr int PITCH = QW * NFACE;          // elements of one shared wave value over the faces
   static constexpr int NQ = ME * QW * QW;           // staged q of the tile and two ghost layers
   static constexpr int NFX = ME * QW * (T + 1);      // fm / fp of every staged row
   static constexpr int NQX = ME * QW * T;            // x-updated q of the tile's columns
   static constexpr int NG = ME * (T + 1) * T;        // gm / gp
-  static constexpr int WREC = MW * ME + MW + 2 * ME;
-  static constexpr int NW = STEP2_RC * (T + 3) * WREC;
+  static constexpr int NX = MW * ME * PITCH;         // waves
   static constexpr int NA = S::NAUX > 0 ? MAXAUX2 : 0;
   static constexpr int NAQ = NA * QW * QW;           // staged aux, [m][b][a] like Qs
-  static constexpr int TOTAL = NQ + 2 * NFX + NQX + 2 * NG + NW + NAQ + 32;
+  static constexpr int TOTAL = NQ + 2 * NFX + NQX + 2 * NG + NX + NAQ + 32;
+  static_assert(PITCH <= SPLIT2_THREADS, "a thread per face of a sweep");
 };
 
+// One round of a split sweep: flux2_dimSplit.f at the faces of the tile's lines. Thread tid
+// takes face ff of its line (active: it exists; flux: it is one of the tile's own), between
+// the cells whose values are ql(m) and qr(m); the faces beside it are threads tid -+ nb.
+template <class S, int IXY, class R, class QL, class QR>
+__device__ __forceinline__ void split2_round(const StepParams& sp, R* X, int pitch, bool active, bool flux, int nb, QL ql, QR qr,
+                                             const AuxCell<S, R>& aL, const AuxCell<S, R>& aR, R dl, R dr, R& cfl,
+                                             R (&fm)[S::MEQN], R (&fp)[S::MEQN]) {
+  constexpr int ME = S::MEQN, MW = S::MWAVES;
+  const int tid = threadIdx.x;
+  R s[MW], amdq[ME], apdq[ME];
+  if (active) {
+    R qL[ME], qR[ME], wave[MW][ME];
+#pragma unroll
+    for (int m = 0; m < ME; ++m) { qL[m] = ql(m); qR[m] = qr(m); }
+    S::template rpn<R>(sp.prob, IXY, qL, qR, aL.v, aR.v, wave, s, amdq, apdq);
+#pragma unroll
+    for (int mw = 0; mw < MW; ++mw)
+#pragma unroll
+      for (int m = 0; m < ME; ++m) X[(mw * ME + m) * pitch + tid] = wave[mw][m];
+    if (flux) {
+#pragma unroll
+      for (int mw = 0; mw < MW; ++mw) cfl = dmax(cfl, dmax(dr * s[mw], -dl * s[mw]));
+    }
+  }
+  __syncthreads();
+  if (flux) {
+    R cq[ME];
+    limited_fluxes<S, R>(sp, X, pitch, tid, nb, dl, dr, s, amdq, apdq, cq, fm, fp);
+  }
+}
+
 template <class S, class R>
-__global__ void __launch_bounds__(STEP2_THREADS) step2s_kernel(StepArgs a) {
+__global__ void __launch_bounds__(SPLIT2_THREADS, std::is_same<S, Euler2>::value && sizeof(R) == 8 ? 1 : 2) step2s_kernel(StepArgs a) {
   using L = Split2Layout<S>;
-  constexpr int ME = L::ME, T = L::T, QW = L::QW, WREC = L::WREC;
+  constexpr int ME = L::ME, T = L::T, QW = L::QW, NFACE = L::NFACE;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* Qs = reinterpret_cast<R*>(smem_raw);
   R* FXm = Qs + L::NQ;
@@ -643,8 +607,8 @@ __global__ void __launch_bounds__(STEP2_THREADS) step2s_kernel(StepArgs a) {
   R* Qx = FXp + L::NFX;
   R* GM = Qx + L::NQX;
   R* GP = GM + L::NG;
-  R* W = GP + L::NG;
-  R* As = W + L::NW;
+  R* X = GP + L::NG;
+  R* As = X + L::NX;
   R* red = As + L::NAQ;
   __shared__ int s_item;
   const int tid = threadIdx.x;
@@ -669,114 +633,94 @@ __global__ void __launch_bounds__(STEP2_THREADS) step2s_kernel(StepArgs a) {
     ++iter;
     if (w >= a.nwork) break;
     const StepWork wk = a.work[w];
-    const PatchDev P = a.patches[wk.patch];
+    const PatchDev& P = a.patches[wk.patch];
+    const int cur = P.cur;
     const int mx = P.ihi - P.ilo + 1, my = P.jhi - P.jlo + 1;
     const int mitot = P.mitot, mjtot = P.mjtot;
     const int i0 = wk.ti0, j0 = wk.tj0;
     const int tw = min(T, mx - i0 + 1), th = min(T, my - j0 + 1);
-    const R* qin = static_cast<const R*>(a.pool) + P.q[P.cur];
-    R* qout = static_cast<R*>(a.pool) + P.q[1 - P.cur];
+    const R* qin = static_cast<const R*>(a.pool) + P.q[cur];
+    R* qout = static_cast<R*>(a.pool) + P.q[1 - cur];
     const long long plane = (long long)mitot * mjtot;
     const int lw = tw + 4, lh = th + 4;
-    for (int it = tid; it < ME * lw * lh; it += STEP2_THREADS) {
-      const int m = it / (lw * lh), rem = it % (lw * lh);
-      const int b = rem / lw, aa = rem % lw;
-      const int ie = (i0 - 2 + aa) + 1, je = (j0 - 2 + b) + 1;
-      Qs[(m * QW + b) * QW + aa] = qin[m * plane + (long long)je * mitot + ie];
-    }
-    if (L::NA > 0) {
-      const R* aux = static_cast<const R*>(a.pool) + P.aux;
-      const int na = min(L::NA, a.sp.prob.naux);
-      for (int it = tid; it < na * lw * lh; it += STEP2_THREADS) {
-        const int m = it / (lw * lh), rem = it % (lw * lh);
-        const int b = rem / lw, aa = rem % lw;
-        const int ie = (i0 - 2 + aa) + 1, je = (j0 - 2 + b) + 1;
-        As[(m * QW + b) * QW + aa] = aux[m * plane + (long long)je * mitot + ie];
-      }
+    const R* aux = L::NA > 0 ? static_cast<const R*>(a.pool) + P.aux : nullptr;
+    const int na = L::NA > 0 ? min(L::NA, a.sp.prob.naux) : 0;
+    for (int it = tid; it < QW * QW; it += SPLIT2_THREADS) {
+      const int aa = it % QW, b = it / QW;
+      if (aa >= lw || b >= lh) continue;
+      const long long at = (long long)((j0 - 2 + b) + 1) * mitot + (i0 - 2 + aa) + 1;
+      R v[ME];
+#pragma unroll
+      for (int m = 0; m < ME; ++m) v[m] = qin[m * plane + at];
+#pragma unroll
+      for (int m = 0; m < ME; ++m) Qs[(m * QW + b) * QW + aa] = v[m];
+      for (int m = 0; m < na; ++m) As[(m * QW + b) * QW + aa] = aux[m * plane + at];
     }
     __syncthreads();
     // step2x.f90: rows b (j = j0-2+b), faces ff (i = i0-1+ff, between staged columns ff, ff+1)
     {
-      const int nfr = tw + 3, nfl = tw + 1;
-      for (int b0 = 0; b0 < lh; b0 += STEP2_RC) {
-        const int nb = min(STEP2_RC, lh - b0);
-        for (int it = tid; it < nb * nfr; it += STEP2_THREADS) {
-          const int rr = it / nfr, ff = it % nfr, b = b0 + rr;
-          R qL[ME], qR[ME];
+      const int b = tid / NFACE, ff = tid % NFACE;
+      const bool active = b < lh && ff < tw + 3, flux = active && ff >= 1 && ff <= tw + 1;
+      AuxCell<S, R> aL, aR;
+      R dl = dtdx, dr = dtdx, fm[ME], fp[ME];
+      if (active) {
+        if (S::NAUX > 0) { aL.load(As, QW, b, ff); aR.load(As, QW, b, ff + 1); }
+        dl = d1d(dtdx, b, ff); dr = d1d(dtdx, b, ff + 1);
+      }
+      split2_round<S, 1, R>(a.sp, X, L::PITCH, active, flux, 1, [&](int m) { return Qs[(m * QW + b) * QW + ff]; },
+                            [&](int m) { return Qs[(m * QW + b) * QW + ff + 1]; }, aL, aR, dl, dr, cfl, fm, fp);
+      if (flux) {
 #pragma unroll
-          for (int m = 0; m < ME; ++m) { qL[m] = Qs[(m * QW + b) * QW + ff]; qR[m] = Qs[(m * QW + b) * QW + ff + 1]; }
-          AuxCell<S, R> aL, aR;
-          if (S::NAUX > 0) { aL.load(As, QW, b, ff); aR.load(As, QW, b, ff + 1); }
-          face_record<S, R>(a.sp, 1, qL, qR, aL.v, aR.v, W + (rr * (T + 3) + ff) * WREC, d1d(dtdx, b, ff),
-                            d1d(dtdx, b, ff + 1), ff >= 1 && ff <= nfl, cfl);
+        for (int m = 0; m < ME; ++m) {
+          FXm[(m * QW + b) * (T + 1) + ff - 1] = fm[m];
+          FXp[(m * QW + b) * (T + 1) + ff - 1] = fp[m];
         }
-        __syncthreads();
-        for (int it = tid; it < nb * nfl; it += STEP2_THREADS) {
-          const int rr = it / nfl, fa = it % nfl, b = b0 + rr;
-          const R* rm = W + (rr * (T + 3) + fa) * WREC;
-          R amdq[ME], apdq[ME], cqxx[ME], fm[ME], fp[ME];
-          face_fluxes<S, R>(a.sp, rm, rm + WREC, rm + 2 * WREC, d1d(dtdx, b, fa + 1), d1d(dtdx, b, fa + 2), amdq, apdq,
-                            cqxx, fm, fp);
-#pragma unroll
-          for (int m = 0; m < ME; ++m) {
-            FXm[(m * QW + b) * (T + 1) + fa] = fm[m];
-            FXp[(m * QW + b) * (T + 1) + fa] = fp[m];
-          }
-        }
-        __syncthreads();
       }
     }
+    __syncthreads();
     // stepgrid_dimSplit.f:88-103: x-update of every staged row's tile cells. The rows that
     // are the patch's ghost rows (below row 1 or above row my) keep their x-updated values
     // in the new store1, as the reference's array does (binary output writes them).
-    for (int it = tid; it < ME * lh * tw; it += STEP2_THREADS) {
-      const int m = it / (lh * tw), rem = it % (lh * tw);
-      const int b = rem / tw, c = rem % tw;
-      const R df = dtdx * (FXm[(m * QW + b) * (T + 1) + c + 1] - FXp[(m * QW + b) * (T + 1) + c]);
-      const R v = Qs[(m * QW + b) * QW + c + 2] - (capa ? df / kap(b, c + 2) : df);
-      Qx[(m * QW + b) * T + c] = v;
+    if (const int c = tid % T, b = tid / T; b < lh && c < tw) {
       const int jrow = j0 - 2 + b;
-      if (jrow < 1 || jrow > my) qout[m * plane + (long long)(jrow + 1) * mitot + (i0 + c + 1)] = v;
+#pragma unroll
+      for (int m = 0; m < ME; ++m) {
+        const R df = dtdx * (FXm[(m * QW + b) * (T + 1) + c + 1] - FXp[(m * QW + b) * (T + 1) + c]);
+        const R v = Qs[(m * QW + b) * QW + c + 2] - (capa ? df / kap(b, c + 2) : df);
+        Qx[(m * QW + b) * T + c] = v;
+        if (jrow < 1 || jrow > my) qout[m * plane + (long long)(jrow + 1) * mitot + (i0 + c + 1)] = v;
+      }
     }
     __syncthreads();
     // step2y.f90: columns c (i = i0+c), faces ff (j = j0-1+ff, between x-updated rows ff, ff+1)
     {
-      const int nfr = th + 3, nfl = th + 1;
-      for (int c0 = 0; c0 < tw; c0 += STEP2_RC) {
-        const int nc = min(STEP2_RC, tw - c0);
-        for (int it = tid; it < nc * nfr; it += STEP2_THREADS) {
-          const int rr = it / nfr, ff = it % nfr, c = c0 + rr;
-          R qL[ME], qR[ME];
+      const int c = tid % T, ff = tid / T;
+      const bool active = c < tw && ff < th + 3, flux = active && ff >= 1 && ff <= th + 1;
+      AuxCell<S, R> aL, aR;
+      R dl = dtdy, dr = dtdy, fm[ME], fp[ME];
+      if (active) {
+        if (S::NAUX > 0) { aL.load(As, QW, ff, c + 2); aR.load(As, QW, ff + 1, c + 2); }
+        dl = d1d(dtdy, ff, c + 2); dr = d1d(dtdy, ff + 1, c + 2);
+      }
+      split2_round<S, 2, R>(a.sp, X, L::PITCH, active, flux, T, [&](int m) { return Qx[(m * QW + ff) * T + c]; },
+                            [&](int m) { return Qx[(m * QW + ff + 1) * T + c]; }, aL, aR, dl, dr, cfl, fm, fp);
+      if (flux) {
 #pragma unroll
-          for (int m = 0; m < ME; ++m) { qL[m] = Qx[(m * QW + ff) * T + c]; qR[m] = Qx[(m * QW + ff + 1) * T + c]; }
-          AuxCell<S, R> aL, aR;
-          if (S::NAUX > 0) { aL.load(As, QW, ff, c + 2); aR.load(As, QW, ff + 1, c + 2); }
-          face_record<S, R>(a.sp, 2, qL, qR, aL.v, aR.v, W + (rr * (T + 3) + ff) * WREC, d1d(dtdy, ff, c + 2),
-                            d1d(dtdy, ff + 1, c + 2), ff >= 1 && ff <= nfl, cfl);
+        for (int m = 0; m < ME; ++m) {
+          GM[(m * (T + 1) + ff - 1) * T + c] = fm[m];
+          GP[(m * (T + 1) + ff - 1) * T + c] = fp[m];
         }
-        __syncthreads();
-        for (int it = tid; it < nc * nfl; it += STEP2_THREADS) {
-          const int rr = it / nfl, fb = it % nfl, c = c0 + rr;
-          const R* rm = W + (rr * (T + 3) + fb) * WREC;
-          R amdq[ME], apdq[ME], cqxx[ME], fm[ME], fp[ME];
-          face_fluxes<S, R>(a.sp, rm, rm + WREC, rm + 2 * WREC, d1d(dtdy, fb + 1, c + 2), d1d(dtdy, fb + 2, c + 2), amdq,
-                            apdq, cqxx, fm, fp);
-#pragma unroll
-          for (int m = 0; m < ME; ++m) {
-            GM[(m * (T + 1) + fb) * T + c] = fm[m];
-            GP[(m * (T + 1) + fb) * T + c] = fp[m];
-          }
-        }
-        __syncthreads();
       }
     }
+    __syncthreads();
     // stepgrid_dimSplit.f:118-133: y-update of the tile's cells into the other buffer
-    for (int it = tid; it < ME * th * tw; it += STEP2_THREADS) {
-      const int m = it / (th * tw), rem = it % (th * tw);
-      const int rb = rem / tw, ca = rem % tw;
-      const R dg = dtdy * (GM[(m * (T + 1) + rb + 1) * T + ca] - GP[(m * (T + 1) + rb) * T + ca]);
-      const R qn = Qx[(m * QW + rb + 2) * T + ca] - (capa ? dg / kap(rb + 2, ca + 2) : dg);
-      qout[m * plane + (long long)(j0 + rb + 1) * mitot + (i0 + ca + 1)] = qn;
+    if (const int ca = tid % T, rb = tid / T; rb < th && ca < tw) {
+#pragma unroll
+      for (int m = 0; m < ME; ++m) {
+        const R dg = dtdy * (GM[(m * (T + 1) + rb + 1) * T + ca] - GP[(m * (T + 1) + rb) * T + ca]);
+        const R qn = Qx[(m * QW + rb + 2) * T + ca] - (capa ? dg / kap(rb + 2, ca + 2) : dg);
+        qout[m * plane + (long long)(j0 + rb + 1) * mitot + (i0 + ca + 1)] = qn;
+      }
     }
     // the tile's own rows start at staged row 2 of FXm / FXp
     register_epilogue<ME, R>(a, wk, P, i0, j0, tw, th, dt, FXm + 2 * (T + 1), FXp + 2 * (T + 1), GM, GP, QW);
@@ -795,7 +739,7 @@ static void launch_step2_t(const StepArgs& a, int grid, cudaStream_t s) {
     }();
     (void)attr;
     if (grid <= 0) return;
-    step2s_kernel<S, R><<<grid, STEP2_THREADS, sm, s>>>(a);
+    step2s_kernel<S, R><<<grid, SPLIT2_THREADS, sm, s>>>(a);
     AMR_CUDA(cudaGetLastError());
     return;
   }

@@ -7,7 +7,7 @@ namespace amrb {
 
 constexpr int TILE2 = 16;      // interior cells per tile side in the 2D patch step
 constexpr int STEP2_THREADS = 352;  // one thread per face of a sweep over a tile: 18 lines of 19 faces, whole warps
-constexpr int STEP2_RC = 6;         // rows per Riemann chunk of the split step
+constexpr int SPLIT2_THREADS = 384;  // the same for the dimensionally split step: 20 rows of 19 faces
 
 // One tile of one patch (the batched path launches all tiles of a level at once).
 struct StepWork {
