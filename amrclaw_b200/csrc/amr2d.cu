@@ -77,7 +77,7 @@ struct FillProg {
   DBuf<FillChunk> d_chunks;
   DBuf<BcOp> d_bcs;
   DBuf<double> d_capa;
-  std::vector<int> ch_lo, ch_hi, bc_lo, bc_hi;
+  std::vector<int> ch_lo, ch_hi, bc_lo, bc_hi, bc_most;
   void clear() {
     rects.clear(); ops.clear(); op_stage.clear(); bcs.clear(); bc_stage.clear(); capa.clear();
     nstages = 0; zero_scratch = false;
@@ -946,12 +946,14 @@ class Amr2Gpu {
     for (size_t i = 0; i < bidx.size(); ++i) bidx[i] = (int)i;
     std::stable_sort(bidx.begin(), bidx.end(), [&](int a, int b) { return P.bc_stage[a] < P.bc_stage[b]; });
     std::vector<BcOp> bcs;
-    P.bc_lo.assign(P.nstages, 0); P.bc_hi.assign(P.nstages, 0);
+    P.bc_lo.assign(P.nstages, 0); P.bc_hi.assign(P.nstages, 0); P.bc_most.assign(P.nstages, 0);
     s = -1;
     for (int k : bidx) {
       const int stg = P.bc_stage[k];
       while (s < stg) { ++s; P.bc_lo[s] = (int)bcs.size(); P.bc_hi[s] = (int)bcs.size(); }
       bcs.push_back(P.bcs[k]);
+      bcs.back().flat = bc_is_flat(P.bcs[k]) ? 1 : 0;
+      P.bc_most[s] = std::max(P.bc_most[s], bc_cells(P.bcs[k]));
       P.bc_hi[s] = (int)bcs.size();
     }
     while (s + 1 < P.nstages) { ++s; P.bc_lo[s] = P.bc_hi[s] = (int)bcs.size(); }
@@ -1010,6 +1012,7 @@ class Amr2Gpu {
         a.rects = X->d_rects.d; a.ops = X->d_ops.d; a.chunks = X->d_chunks.d + X->ch_lo[s]; a.nchunks = X->ch_hi[s] - X->ch_lo[s];
         if (k == 0) { a.modes = modes; a.modes_dev = modes_dev; }
         b.rects = X->d_rects.d; b.ops = X->d_bcs.d + X->bc_lo[s]; b.nops = X->bc_hi[s] - X->bc_lo[s];
+        b.max_cells = X->bc_most[s];
       }
       if (fa[0].nchunks + fa[1].nchunks > 0) { launch_fill_pair(fa[0], fa[1], st, f32); ++nkernels; }
       if (ba[0].nops + ba[1].nops > 0) { launch_bc_pair(ba[0], ba[1], st, f32); ++nkernels; }

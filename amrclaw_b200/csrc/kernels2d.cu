@@ -993,7 +993,7 @@ void launch_fill_pair(const FillArgs& a, const FillArgs& b, cudaStream_t s, bool
 
 // phase 0: x-sides over all rows; phase 1: y-sides over all columns (after phase 0)
 template <class T>
-__device__ __forceinline__ void bc_op(const BcArgs& a, int op, int phase) {
+__device__ __forceinline__ void bc_op(const BcArgs& a, int op, int phase, int nblocks) {
   const BcOp o = a.ops[op];
   T* v; int nrow = o.nrow, ncol = o.ncol;
   if (o.dst_patch >= 0) { const PatchDev& P = a.patches[o.dst_patch]; v = static_cast<T*>(a.pool) + P.q[P.cur]; }
@@ -1005,7 +1005,7 @@ __device__ __forceinline__ void bc_op(const BcArgs& a, int op, int phase) {
     const int nl = (o.nxl > 0 && (o.bxl == 1 || o.bxl == 3)) ? o.nxl : 0;
     const int nr = (o.ibeg > 0 && (o.bxr == 1 || o.bxr == 3)) ? nrow - o.ibeg + 1 : 0;
     const int tot = (nl + nr) * ncol;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += gridDim.x * blockDim.x) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += nblocks * blockDim.x) {
       const int j = t / (nl + nr) + 1, k = t % (nl + nr);
       if (k < nl) {
         const int i = k + 1;
@@ -1023,7 +1023,7 @@ __device__ __forceinline__ void bc_op(const BcArgs& a, int op, int phase) {
     const int nb = (o.nyb > 0 && (o.byl == 1 || o.byl == 3)) ? o.nyb : 0;
     const int nt = (o.jbeg > 0 && (o.byr == 1 || o.byr == 3)) ? ncol - o.jbeg + 1 : 0;
     const int tot = (nb + nt) * nrow;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += gridDim.x * blockDim.x) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += nblocks * blockDim.x) {
       const int i = t % nrow + 1, k = t / nrow;
       if (k < nb) {
         const int j = k + 1;
@@ -1044,20 +1044,62 @@ template <class T>
 __global__ void bc_kernel(BcArgs a, int phase) {
   const int op = blockIdx.y;
   if (op >= a.nops) return;
-  bc_op<T>(a, op, phase);
+  bc_op<T>(a, op, phase, gridDim.x);
 }
-// the ops of two independent programs, one block per op doing phase 0 then phase 1 (the
-// y-sides read the corners the x-sides wrote; each op has its own destination array)
+// Both phases of one op in one pass over its ghost cells, a thread per (component, cell): a
+// cell beyond an x side takes the value at its source column, one beyond a y side at its
+// source row, and a corner at both, which is what the y phase copies there after the x phase.
+// The sources are cells that the op does not write (BcOp::flat).
 template <class T>
-__global__ void bc_pair_kernel(BcArgs a, BcArgs b) {
+__device__ __forceinline__ void bc_flat(const BcArgs& a, const BcOp& o) {
+  const int nrow = o.nrow, ncol = o.ncol;
+  T* v;
+  if (o.dst_patch >= 0) { const PatchDev& P = a.patches[o.dst_patch]; v = static_cast<T*>(a.pool) + P.q[P.cur]; }
+  else v = static_cast<T*>(a.pool) + a.rects[o.dst_rect].off;
+  const int nl = bc_set(o.bxl) ? o.nxl : 0, nr = o.ibeg > 0 && bc_set(o.bxr) ? nrow - o.ibeg + 1 : 0;
+  const int nb = bc_set(o.byl) ? o.nyb : 0, nt = o.jbeg > 0 && bc_set(o.byr) ? ncol - o.jbeg + 1 : 0;
+  const int nx = nl + nr, ny = nb + nt, mid = nrow - nx;
+  const int tx = nx * ncol, tot = tx + ny * mid;
+  const long long plane = (long long)nrow * ncol;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < tot * a.nvar; t += gridDim.x * blockDim.x) {
+    const int m = t / tot, c = t - m * tot;
+    int i, j;  // 1-based
+    if (c < tx) {
+      const int k = c % nx;
+      j = c / nx + 1;
+      i = k < nl ? k + 1 : o.ibeg + (k - nl);
+    } else {
+      const int k = (c - tx) / mid;
+      i = nl + (c - tx) % mid + 1;
+      j = k < nb ? k + 1 : o.jbeg + (k - nb);
+    }
+    int si = i, sj = j;
+    bool neg = false;
+    if (i <= nl) { si = o.bxl == 1 ? o.nxl + 1 : 2 * o.nxl + 1 - i; neg = o.bxl == 3 && m == 1; }
+    else if (nr > 0 && i >= o.ibeg) { si = o.bxr == 1 ? o.ibeg - 1 : 2 * o.ibeg - 1 - i; neg = o.bxr == 3 && m == 1; }
+    if (j <= nb) { sj = o.byl == 1 ? o.nyb + 1 : 2 * o.nyb + 1 - j; neg = neg || (o.byl == 3 && m == 2); }
+    else if (nt > 0 && j >= o.jbeg) { sj = o.byr == 1 ? o.jbeg - 1 : 2 * o.jbeg - 1 - j; neg = neg || (o.byr == 3 && m == 2); }
+    const T x = v[m * plane + (long long)(sj - 1) * nrow + (si - 1)];
+    v[m * plane + (long long)(j - 1) * nrow + (i - 1)] = neg ? -x : x;
+  }
+}
+// The ops of two independent programs: a row of blocks per op. An op too narrow for one pass
+// (a source of one side is a ghost of another) is left to its first block, which does the x
+// phase and then the y phase.
+// One block per op with a chain of load, store, load for every component took 150 us for the
+// four sides of a 1002^2 grid and 5.6 us for the small patches of an adaptive run.
+template <class T>
+__global__ void __launch_bounds__(128) bc_pair_kernel(BcArgs a, BcArgs b) {
   const int op = blockIdx.y;
   const bool first = op < a.nops;
   const BcArgs& A = first ? a : b;
   const int o = first ? op : op - a.nops;
   if (o >= A.nops) return;
-  bc_op<T>(A, o, 0);
+  if (A.ops[o].flat) { bc_flat<T>(A, A.ops[o]); return; }
+  if (blockIdx.x != 0) return;
+  bc_op<T>(A, o, 0, 1);
   __syncthreads();
-  bc_op<T>(A, o, 1);
+  bc_op<T>(A, o, 1, 1);
 }
 void launch_bc_pair(const BcArgs& a, const BcArgs& b, cudaStream_t s, bool f32) {
   const int n = a.nops + b.nops;
@@ -1070,8 +1112,10 @@ void launch_bc_pair(const BcArgs& a, const BcArgs& b, cudaStream_t s, bool f32) 
     }
     return;
   }
-  if (f32) bc_pair_kernel<float><<<dim3(1, n), 128, 0, s>>>(a, b);
-  else bc_pair_kernel<double><<<dim3(1, n), 128, 0, s>>>(a, b);
+  const long long items = (long long)std::max(a.max_cells, b.max_cells) * std::max(a.nvar, b.nvar);
+  const int bx = (int)std::max<long long>(1, std::min<long long>((items + 127) / 128, 256));
+  if (f32) bc_pair_kernel<float><<<dim3(bx, n), 128, 0, s>>>(a, b);
+  else bc_pair_kernel<double><<<dim3(bx, n), 128, 0, s>>>(a, b);
   AMR_CUDA(cudaGetLastError());
 }
 void launch_bc(const BcArgs& a, int phase, cudaStream_t s, bool f32) {

@@ -102,7 +102,29 @@ struct BcOp {
   int nrow, ncol;
   int nxl, ibeg, nyb, jbeg;      // ghost extents (0: side not outside the domain)
   int bxl, bxr, byl, byr;        // boundary codes (1 extrap, 3 wall, 0/2 none)
+  int flat;                      // 1: every source is a cell the op does not write (bc_is_flat)
 };
+// whether a side with this code is set by bc2amr (else its cells are left as they are)
+__host__ __device__ constexpr bool bc_set(int code) { return code == 1 || code == 3; }
+// The sources of each axis are interior cells of the array: the low side's lie between its
+// ghosts and the high side's, and the other way round.
+__host__ __device__ inline bool bc_axis_flat(int n, int lo, int codel, int beg, int codeh) {
+  const int nl = bc_set(codel) ? lo : 0, first = nl + 1, last = beg > 0 && bc_set(codeh) ? beg - 1 : n;
+  if (first > last) return false;
+  // (an inactive side takes no sources; its cells may serve the other side)
+  if (nl > 0 && codel == 3 && 2 * nl > last) return false;
+  if (last < n && codeh == 3 && 2 * beg - 1 - n < first) return false;
+  return true;
+}
+__host__ __device__ inline bool bc_is_flat(const BcOp& o) {
+  return bc_axis_flat(o.nrow, o.nxl, o.bxl, o.ibeg, o.bxr) && bc_axis_flat(o.ncol, o.nyb, o.byl, o.jbeg, o.byr);
+}
+// ghost cells the op sets
+__host__ __device__ inline int bc_cells(const BcOp& o) {
+  const int nx = (bc_set(o.bxl) ? o.nxl : 0) + (o.ibeg > 0 && bc_set(o.bxr) ? o.nrow - o.ibeg + 1 : 0);
+  const int ny = (bc_set(o.byl) ? o.nyb : 0) + (o.jbeg > 0 && bc_set(o.byr) ? o.ncol - o.jbeg + 1 : 0);
+  return nx * o.ncol + ny * (o.nrow - nx);
+}
 
 struct FillArgs {
   void* pool;
@@ -128,6 +150,7 @@ struct BcArgs {
   const BcOp* ops;
   int nops;
   int nvar;
+  int max_cells;             // most ghost cells of an op (sizes the launch of a pair)
 };
 
 // ---------------------------------------------------------------- registers, update
