@@ -18,6 +18,7 @@
 #include "params.hpp"
 #include "cluster2d.hpp"
 #include "flags3d.cuh"
+#include "bisect.hpp"
 #include "gridindex.hpp"
 #include "workpool.hpp"
 #include "noalloc2d.cuh"
@@ -213,6 +214,7 @@ class Amr2Gpu {
     pool.destroy(); regs.destroy();
     if (st) cudaStreamSynchronize(st);
     stg.destroy();
+    bis.free(); sig_mask.free(); sig_pts.free(); sig_off.free(); sig_hist.free(); sig_boxes.free();
     d_patches.free(); d_gauge_out.free(); fl_out.free(); fl_off.free(); fl_pl.free();
     if (d_cfl) cudaFree(d_cfl);
     if (d_mass) cudaFree(d_mass);
@@ -2077,11 +2079,25 @@ class Amr2Gpu {
   DBuf<int> sig_pts, sig_off, sig_hist;
   DBuf<SigBox> sig_boxes;
   LvlDims sig_dims{0, 0, 1};
+  DeviceBisect bis;
+  const std::vector<Pt>* sig_points = nullptr;  // points still to be scattered to sig_mask (grdfit holds them)
+  // the level's points as a one-plane flag array, once per bisection and only where a wave needs it
+  void scatter_points() {
+    if (!sig_points) return;
+    sig_mask.ensure((size_t)sig_dims.size());
+    std::vector<int> flat(2 * sig_points->size());
+    for (size_t k = 0; k < sig_points->size(); ++k) { flat[2 * k] = (*sig_points)[k].i; flat[2 * k + 1] = (*sig_points)[k].j; }
+    sig_pts.upload(flat, st, stg);
+    launch_scatter_points2(sig_pts.d, (int)sig_points->size(), sig_mask.d, sig_dims, st);
+    ++nkernels;
+    sig_points = nullptr;
+  }
   // signs.f on the device for the boxes of clus (1-based array indices = level index + 1);
   // fills n, lo, hi; si / sj (optional): each cluster's counts at 1-based level positions
   void signatures(std::vector<Clu2>& clus, std::vector<std::vector<int>>* si, std::vector<std::vector<int>>* sj) {
     const int nb = (int)clus.size();
     if (nb == 0) return;
+    scatter_points();
     std::vector<SigBox> bx(nb);
     std::vector<int> off(nb + 1, 0);
     int maxlen = 0;
@@ -2127,16 +2143,27 @@ class Amr2Gpu {
     rect[0] = c.lo[0] - 1; rect[1] = c.hi[0] - 1; rect[2] = c.lo[1] - 1; rect[3] = c.hi[1] - 1;
     return (double)c.n / (double)((rect[1] - rect[0] + 1) * (rect[3] - rect[2] + 1));
   }
-  // smartbis.f, breadth first over the device signatures; leaves in the reference's order
-  // (the part at or above the cut first)
+  // smartbis.f in one launch (DeviceBisect); past its limits breadth first over the device
+  // signatures. Leaves in the reference's order (the part at or above the cut first)
   std::vector<Clu2> bisect_on_device(const std::vector<Pt>& pts, int lcheck, double cutoff) {
     sig_dims = LvlDims{iregsz[lcheck], jregsz[lcheck], 1};
-    sig_mask.ensure((size_t)sig_dims.size());
-    std::vector<int> flat(2 * pts.size());
-    for (size_t k = 0; k < pts.size(); ++k) { flat[2 * k] = pts[k].i; flat[2 * k + 1] = pts[k].j; }
-    sig_pts.upload(flat, st, stg);
-    launch_scatter_points2(sig_pts.d, (int)pts.size(), sig_mask.d, sig_dims, st);
-    ++nkernels;
+    sig_points = &pts;
+    std::vector<unsigned long long> list(pts.size());
+    for (size_t k = 0; k < pts.size(); ++k) list[k] = bisect_point(pts[k].i + 1, pts[k].j + 1, 1);
+    std::vector<BisectNode> tree;
+    nkernels += 2;
+    if (bis.run(2, nullptr, sig_dims, list, cutoff, st, stg, tree)) {
+      std::vector<Clu2> out;
+      for (int id : DeviceBisect::leaves(tree)) {
+        const BisectNode& N = tree[id];
+        Clu2 c;
+        c.n = N.n;
+        for (int d = 0; d < 3; ++d) { c.box.lo[d] = N.lo[d]; c.box.hi[d] = N.hi[d]; }
+        for (int d = 0; d < 2; ++d) { c.lo[d] = N.clo[d]; c.hi[d] = N.chi[d]; }
+        out.push_back(c);
+      }
+      return out;
+    }
     struct Node { Clu2 c; int child = -1; };
     std::vector<Node> T(1);
     T[0].c.box = SigBox{{1, 1, 1}, {sig_dims.is, sig_dims.js, 1}};
@@ -2237,6 +2264,7 @@ class Amr2Gpu {
       prv = mnew;
       ++icl;
     }
+    sig_points = nullptr;
     birect(newstl[levnew]);
     tr_cluster += std::chrono::duration<double>(std::chrono::steady_clock::now() - tc0).count();
   }

@@ -13,6 +13,7 @@
 // grdfit.f, birect.f, gfixup.f, filval.f) with the gradient test on the device.
 #include "kernels3d.cuh"
 #include "flags3d.cuh"
+#include "bisect.hpp"
 #include "valout.hpp"
 #include "params.hpp"
 #include "gridindex.hpp"
@@ -241,6 +242,7 @@ class Amr3Gpu : public AmrSolver {
     stg.destroy();
     d_patches.free(); d_stash.free(); d_flux.free(); d_split.free(); d_gauge_out.free(); d_aux_jobs.free(); d_aux_fac.free();
     for (DBuf<int8_t>* b : {&lv_a, &lv_b, &lv_n, &lv_t1, &lv_t2}) b->free();
+    bis.free();
     lv_boxes.free(); lv_proj.free(); lv_c0.free(); lv_plist.free();
     if (lv_host) cudaFreeHost(lv_host);
     if (d_cfl) cudaFree(d_cfl);
@@ -2067,11 +2069,26 @@ class Amr3Gpu : public AmrSolver {
     iside = lv[0][1];
     if (lv[0][0] < 2) index = 0;
   }
-  // smartbis.f: bisect until every cluster's efficiency reaches cutoff or it has no cut;
-  // breadth first (one signature wave per depth), then the leaves in the reference's
+  // smartbis.f: bisect until every cluster's efficiency reaches cutoff or it has no cut, in
+  // one launch (DeviceBisect); past its limits breadth first here, one signature wave per
+  // depth, then the leaves in the reference's
   // depth-first order: the part at or above the cut before the part below it
+  DeviceBisect bis;
   std::vector<Clu3> cluster_on_device(double cutoff) {
     const int dims[3] = {lv_dims.is, lv_dims.js, lv_dims.ks};
+    std::vector<BisectNode> tree;
+    nkernels += 3;
+    if (bis.run(3, lv_b.d, lv_dims, {}, cutoff, st, stg, tree)) {
+      std::vector<Clu3> out;
+      for (int id : DeviceBisect::leaves(tree)) {
+        const BisectNode& N = tree[id];
+        Clu3 c;
+        c.n = N.n;
+        for (int d = 0; d < 3; ++d) { c.box.lo[d] = N.lo[d]; c.box.hi[d] = N.hi[d]; c.lo[d] = N.clo[d]; c.hi[d] = N.chi[d]; }
+        out.push_back(c);
+      }
+      return out;
+    }
     struct Node { Clu3 c; int child = -1; };  // child: the upper part; child+1 the lower part
     std::vector<Node> T(1);
     T[0].c.box = SigBox{{1, 1, 1}, {dims[0], dims[1], dims[2]}};

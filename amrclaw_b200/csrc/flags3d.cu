@@ -407,6 +407,324 @@ void launch_signatures3(const int8_t* f, LvlDims d, const SigBox* boxes, int nbo
   AMR_CUDA(cudaGetLastError());
 }
 
+// ======================================================================= bisection
+namespace {
+constexpr int BIS_THREADS = 1024;
+constexpr int BIS_BLOCKS = 32;
+constexpr int BIS_Q = 4;     // points of a thread in flight
+constexpr int BIS_SH = 320;  // counts of a node that its warp keeps in shared memory
+
+__global__ void bisect_head_kernel(BisectHead* h, unsigned npts) {
+  *h = BisectHead{};
+  h->points = npts;
+}
+// the flagged cells of the interior, in any order (only their counts are used)
+__global__ void __launch_bounds__(256) list_points_kernel(const int8_t* f, LvlDims d, unsigned long long* pts, unsigned max_points, BisectHead* h) {
+  const long long row = (d.is + 31) / 32 * 32, n = row * d.js * d.ks;  // whole warps per i-row
+  const int lane = threadIdx.x & 31;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(t % row) + 1;
+    const long long r = t / row;
+    const int j = (int)(r % d.js) + 1, k = (int)(r / d.js) + 1;
+    const bool on = i <= d.is && f[d.at(i, j, k)] != 0;
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (m == 0) continue;
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(&h->points, (unsigned)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const unsigned at = base + __popc(m & ((1u << lane) - 1u));
+    if (on && at < max_points) pts[at] = bisect_point(i, j, k);
+  }
+}
+
+// All blocks of the launch (co-resident: it is a cooperative one). False when a block gave up
+// waiting after about a second; every block then leaves.
+__device__ __forceinline__ bool bisect_barrier(BisectHead* h, unsigned& turn) {
+  if (gridDim.x == 1) { __syncthreads(); return true; }
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ++turn;
+    __threadfence();
+    atomicAdd(&h->arrived, 1u);
+    const long long t0 = clock64();
+    ok = 1;
+    while (*(volatile unsigned*)&h->arrived < turn * gridDim.x) {
+      if (clock64() - t0 > 2000000000LL) { ok = 0; break; }
+    }
+    if (!ok) atomicExch(&h->stop, 2);
+    __threadfence();
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// A warp's reduction of a key to its largest, on every lane.
+__device__ __forceinline__ unsigned long long warp_max64(unsigned long long v) {
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = w > v ? w : v;
+  }
+  return v;
+}
+
+// moment.f and findcut.f for one node by one warp, from its counts h (per i, then j, then k).
+// Returns whether it is cut. SH: the counts are in shared memory.
+template <int ND, bool SH>
+__device__ __forceinline__ bool bisect_node(BisectNode& N, const int* h, double cutoff) {
+  const int lane = threadIdx.x & 31;
+  auto at_ = [](const int* q) { return SH ? *q : __ldcg(q); };
+  const int* hd[3];
+  int n = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    hd[d] = h;
+    if (d >= ND) { N.clo[d] = N.lo[d]; N.chi[d] = N.hi[d]; continue; }
+    const int len = N.hi[d] - N.lo[d] + 1;
+    int first = 0x7fffffff, last = -1, sum = 0;
+#pragma unroll 4
+    for (int t = lane; t < len; t += 32) {
+      const int v = at_(h + t);
+      if (v) { first = min(first, t); last = max(last, t); sum += v; }
+    }
+    first = __reduce_min_sync(0xffffffffu, first);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (d == 0) n = __reduce_add_sync(0xffffffffu, sum);
+    N.clo[d] = last < 0 ? N.lo[d] : N.lo[d] + first;
+    N.chi[d] = last < 0 ? N.hi[d] : N.lo[d] + last;
+    h += len;
+  }
+  N.n = n;
+  if (n == 0) return false;
+  int vol = 1;
+#pragma unroll
+  for (int d = 0; d < ND; ++d) vol *= N.chi[d] - N.clo[d] + 1;
+  if ((double)n / (double)vol >= cutoff) return false;
+  // a hole: the first zero of the first direction that has one
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    int z = 0x7fffffff;
+#pragma unroll 4
+    for (int t = N.clo[d] + lane; t <= N.chi[d]; t += 32)
+      if (at_(hd[d] + (t - N.lo[d])) == 0) z = min(z, t);
+    z = __reduce_min_sync(0xffffffffu, z);
+    if (z != 0x7fffffff) { N.dir = d + 1; N.cut = z; return true; }
+  }
+  // the largest sign change of the Laplacian of each direction's counts, the one nearest to
+  // the middle among equals, the first among those
+  int best[3] = {0, 0, 0}, at[3] = {0, 0, 0}, mid[3] = {0, 0, 0};
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    const int lo = N.clo[d], hi = N.chi[d];
+    mid[d] = (lo + hi) / 2;
+    unsigned long long key = 0;
+#pragma unroll 2
+    for (int t = lo + 2 + lane; t <= hi - 1; t += 32) {
+      const int* c = hd[d] + (t - N.lo[d]);
+      const int c0 = at_(c - 2), c1 = at_(c - 1), c2 = at_(c), c3 = at_(c + 1);
+      const int a = c2 - 2 * c1 + c0, b = c3 - 2 * c2 + c1;
+      if (a * b < 0) {
+        const unsigned long long v = ((unsigned long long)abs(a - b) << 42) | ((unsigned long long)(0x1fffff - abs(t - mid[d])) << 21) |
+                                     (unsigned long long)(0x1fffff - t);
+        key = v > key ? v : key;
+      }
+    }
+    key = warp_max64(key);
+    if (key) { best[d] = (int)(key >> 42); at[d] = 0x1fffff - (int)(key & 0x1fffff); }
+  }
+  int index, side;
+  if (ND == 2) {
+    // src/2d/findcut.f: the larger change; of equal ones the one nearer to its middle
+    const bool x = best[0] > best[1] || (best[0] == best[1] && abs(at[0] - mid[0]) < abs(at[1] - mid[1]));
+    side = x ? 1 : 2;
+    index = x ? at[0] : at[1];
+    if ((x ? best[0] : best[1]) < 2) index = 0;
+  } else {
+    // src/3d/findcut.f: the directions ordered by their change, the leading equal ones again
+    // by the distance from their middles
+    int o[3] = {0, 1, 2};
+    for (int a = 0; a < 2; ++a)
+      for (int b = a + 1; b < 3; ++b)
+        if (best[o[a]] < best[o[b]]) { const int t = o[a]; o[a] = o[b]; o[b] = t; }
+    const int same = best[o[0]] > best[o[1]] ? 1 : best[o[1]] > best[o[2]] ? 2 : 3;
+    if (same != 1)
+      for (int a = 0; a < same - 1; ++a)
+        for (int b = a + 1; b < same; ++b)
+          if (abs(at[o[a]] - mid[o[a]]) > abs(at[o[b]] - mid[o[b]])) { const int t = o[a]; o[a] = o[b]; o[b] = t; }
+    index = at[o[0]];
+    side = o[0] + 1;
+    if (best[o[0]] < 2) index = 0;
+  }
+  N.dir = side;
+  N.cut = index;
+  return index != 0;
+}
+
+// One launch for the whole bisection. A wave is the nodes [w0, w1) of one depth: every point
+// moves to its part of the node that was cut above it and counts itself there, then a warp
+// per node takes the decisions that the host took from the counts of a wave, and makes the
+// two parts. Going back to the host between waves cost 24-33 us a wave (an upload, a clear, a
+// launch, a copy and a wait): 205 us a bisection of a 100^2 quadrants run (140 bisections,
+// about 6 waves each), where this launch takes 65 us and is bound by the latency of its waves'
+// dependent L2 reads.
+template <int ND>
+__global__ void __launch_bounds__(BIS_THREADS) bisect_kernel(BisectArgs A) {
+  __shared__ int counts[BIS_THREADS / 32 * BIS_SH];
+  BisectHead* H = A.head;
+  const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31;
+  const unsigned warp = tid >> 5, nwarps = nthr >> 5;
+  unsigned turn = 0;
+  const unsigned np = H->points;
+  if (np > A.max_points) {
+    if (tid == 0) H->stop = 1;
+    return;
+  }
+  const int root_len = A.dims[0] + A.dims[1] + (ND == 3 ? A.dims[2] : 0);
+  for (unsigned t = tid; t < (unsigned)root_len; t += nthr) A.hist[t] = 0;
+  for (unsigned q = tid; q < np; q += nthr) A.node_of[q] = 0;
+  if (tid == 0) {
+    BisectNode R{};
+    for (int d = 0; d < 3; ++d) { R.lo[d] = 1; R.hi[d] = d < ND ? A.dims[d] : 1; }
+    R.child = -1;
+    A.nodes[0] = R;
+    H->nodes = 1;
+  }
+  if (!bisect_barrier(H, turn)) return;
+  int w0 = 0, w1 = 1, cur = 0;
+  while (true) {
+    if (tid == 0) H->hlen[cur ^ 1] = 0;
+    int* hist = A.hist + (long long)cur * A.max_hist;
+    // BIS_Q points of a thread at a time: their loads are in flight together
+    for (unsigned q0 = tid; q0 < np; q0 += BIS_Q * nthr) {
+      unsigned long long P[BIS_Q];
+      int b[BIS_Q], ch[BIS_Q], dir[BIS_Q], cut[BIS_Q], at[BIS_Q], lo[BIS_Q][ND], hi[BIS_Q][ND];
+#pragma unroll
+      for (int u = 0; u < BIS_Q; ++u) {
+        const unsigned q = q0 + u * nthr;
+        b[u] = q < np ? A.node_of[q] : -1;
+        P[u] = q < np ? A.pts[q] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < BIS_Q; ++u) {
+        ch[u] = -2;  // stays where it is
+        if (b[u] < 0 || b[u] >= w0) continue;
+        const BisectNode* N = A.nodes + b[u];
+        ch[u] = __ldcg(&N->child); dir[u] = __ldcg(&N->dir); cut[u] = __ldcg(&N->cut);
+      }
+#pragma unroll
+      for (int u = 0; u < BIS_Q; ++u) {
+        if (ch[u] == -1) b[u] = -1;  // in a leaf
+        if (ch[u] >= 0) {
+          b[u] = (int)((P[u] >> (21 * (dir[u] - 1))) & 0x1fffff) >= cut[u] ? ch[u] : ch[u] + 1;
+          A.node_of[q0 + u * nthr] = b[u];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < BIS_Q; ++u) {
+        if (b[u] < 0) continue;
+        const BisectNode* N = A.nodes + b[u];
+        at[u] = __ldcg(&N->hoff);
+#pragma unroll
+        for (int d = 0; d < ND; ++d) { lo[u][d] = __ldcg(&N->lo[d]); hi[u][d] = __ldcg(&N->hi[d]); }
+      }
+#pragma unroll
+      for (int u = 0; u < BIS_Q; ++u) {
+        if (b[u] < 0) continue;
+        int o = at[u];
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+          atomicAdd(hist + o + ((int)((P[u] >> (21 * d)) & 0x1fffff) - lo[u][d]), 1);
+          o += hi[u][d] - lo[u][d] + 1;
+        }
+      }
+    }
+    if (!bisect_barrier(H, turn)) return;
+    int* next = A.hist + (long long)(cur ^ 1) * A.max_hist;
+    for (int b = w0 + (int)warp; b < w1; b += (int)nwarps) {
+      BisectNode N;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) { N.lo[d] = __ldcg(&A.nodes[b].lo[d]); N.hi[d] = __ldcg(&A.nodes[b].hi[d]); }
+      N.hoff = __ldcg(&A.nodes[b].hoff);
+      N.child = -1; N.dir = 0; N.cut = 0; N.pad = 0;
+      int len_all = 0;
+#pragma unroll
+      for (int d = 0; d < ND; ++d) len_all += N.hi[d] - N.lo[d] + 1;
+      bool cutit;
+      if (len_all <= BIS_SH) {
+        int* own = counts + (threadIdx.x >> 5) * BIS_SH;
+        __syncwarp();
+#pragma unroll 4
+        for (int t = lane; t < len_all; t += 32) own[t] = __ldcg(hist + N.hoff + t);
+        __syncwarp();
+        cutit = bisect_node<ND, true>(N, own, A.cutoff);
+      } else {
+        cutit = bisect_node<ND, false>(N, hist + N.hoff, A.cutoff);
+      }
+      int id = -1, off = 0, len[2] = {0, 0};
+      if (cutit) {
+        int all = 0;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) all += N.chi[d] - N.clo[d] + 1;
+        len[0] = all - (N.cut - N.clo[N.dir - 1]);
+        len[1] = all - (N.chi[N.dir - 1] - N.cut + 1);
+        if (lane == 0) {
+          id = atomicAdd(&H->nodes, 2);
+          off = atomicAdd(&H->hlen[cur ^ 1], len[0] + len[1]);
+        }
+        id = __shfl_sync(0xffffffffu, id, 0);
+        off = __shfl_sync(0xffffffffu, off, 0);
+        if (id + 2 > A.max_nodes || off + len[0] + len[1] > A.max_hist) {
+          if (lane == 0) atomicExch(&H->stop, 1);
+          id = -1;
+        }
+      }
+      if (id >= 0) {
+        for (int t = lane; t < len[0] + len[1]; t += 32) next[off + t] = 0;
+        if (lane == 0) {
+          N.child = id;
+          BisectNode U{};
+#pragma unroll
+          for (int d = 0; d < 3; ++d) { U.lo[d] = N.clo[d]; U.hi[d] = N.chi[d]; }
+          U.child = -1;
+          BisectNode L = U;
+          U.lo[N.dir - 1] = N.cut; U.hoff = off;
+          L.hi[N.dir - 1] = N.cut - 1; L.hoff = off + len[0];
+          A.nodes[id] = U;
+          A.nodes[id + 1] = L;
+        }
+      }
+      if (lane == 0) A.nodes[b] = N;
+    }
+    if (!bisect_barrier(H, turn)) return;
+    if (*(volatile int*)&H->stop) return;
+    w0 = w1;
+    w1 = *(volatile int*)&H->nodes;
+    if (w0 == w1) return;
+    cur ^= 1;
+  }
+}
+}  // namespace
+
+void launch_bisect(int ndim, const BisectArgs& a, const int8_t* f, LvlDims d, unsigned npts, cudaStream_t s) {
+  bisect_head_kernel<<<1, 1, 0, s>>>(a.head, ndim == 3 ? 0u : npts);
+  if (ndim == 3) {
+    const long long cells = (long long)((d.is + 31) / 32 * 32) * d.js * d.ks;
+    list_points_kernel<<<blocks_for(cells, 256), 256, 0, s>>>(f, d, a.pts, a.max_points, a.head);
+  }
+  AMR_CUDA(cudaGetLastError());
+  // a list of up to a few thousand points is one block's work, with no grid barrier
+  const unsigned blocks = ndim == 3 ? BIS_BLOCKS : std::max(1u, std::min((unsigned)BIS_BLOCKS, npts / 4096));
+  if (blocks == 1) {
+    bisect_kernel<2><<<1, BIS_THREADS, 0, s>>>(a);
+    AMR_CUDA(cudaGetLastError());
+    return;
+  }
+  void* args[1] = {const_cast<BisectArgs*>(&a)};
+  AMR_CUDA(cudaLaunchCooperativeKernel(ndim == 3 ? (const void*)bisect_kernel<3> : (const void*)bisect_kernel<2>, dim3(blocks),
+                                       dim3(BIS_THREADS), args, 0, s));
+}
+
 // ======================================================================= Richardson estimation
 namespace {
 template <class T>

@@ -49,6 +49,41 @@ struct SigBox { int lo[3], hi[3]; };
 // hist; maxlen: the largest ni+nj+nk; maxrows: the largest nj*nk (i-rows of a box).
 void launch_signatures3(const int8_t* f, LvlDims d, const SigBox* boxes, int nbox, const int* off, int total, int maxlen,
                         long long maxrows, int* hist, cudaStream_t s);
+// ---- Berger-Rigoutsos bisection as one launch (smartbis.f:25-177 over signs.f, moment.f and
+// findcut.f). A node is a cluster: its box, the count and bounding box of its points, and its
+// cut (dir 1..3, cut: first index of the upper part) with the node of the upper part in
+// `child` and of the lower part in child + 1; child < 0: a leaf. Nodes come breadth first.
+struct BisectNode {
+  int lo[3], hi[3];    // box (1-based level-array indices, inclusive)
+  int clo[3], chi[3];  // bounding box of the points
+  int n, child, dir, cut, hoff, pad;
+};
+struct BisectHead {
+  int nodes;           // nodes made
+  int stop;            // 0: done; else the limits or a wait ran out, and the host bisects by waves
+  unsigned points;     // points of the list
+  unsigned arrived;    // blocks at the grid barrier, counted up
+  int hlen[2];         // histogram ints given out, per buffer
+  int pad[2];
+};
+constexpr int BISECT_FIRST = 512;  // nodes that come back with the first copy
+// Point of the list: 1-based level-array indices, 21 bits each.
+__host__ __device__ inline unsigned long long bisect_point(int i, int j, int k) {
+  return (unsigned long long)i | ((unsigned long long)j << 21) | ((unsigned long long)k << 42);
+}
+struct BisectArgs {
+  BisectHead* head;             // zeroed by the launch; head->points set for a given list
+  BisectNode* nodes; int max_nodes;
+  unsigned long long* pts; unsigned max_points;
+  int* node_of;                 // [max_points]
+  int* hist; int max_hist;      // two buffers of max_hist ints
+  int dims[3];
+  double cutoff;
+};
+// ndim 3: the points are the flagged cells (f != 0) of the level array's interior, listed on
+// the device first; ndim 2: npts points are already in a.pts.
+void launch_bisect(int ndim, const BisectArgs& a, const int8_t* f, LvlDims d, unsigned npts, cudaStream_t s);
+
 // 2D: the level's flag array as a one-plane array (d.ks = 1): zeroed, then 1 at every point
 // (pts: n pairs of 0-based level indices i, j) at array position (i+1, j+1, 1)
 void launch_scatter_points2(const int* pts, int n, int8_t* f, LvlDims d, cudaStream_t s);
