@@ -389,16 +389,15 @@ __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, 
 #pragma unroll
       for (int k = 0; k < NW; ++k) {
         if (sp.mthlim[k] == 0) continue;
-        T dl = T(0), dr = T(0), wn = T(0);
+        // the ratio takes the neighbour on the upwind side
+        const int up = S[k] > T(0) ? l - 1 : l + 1;
+        T dot = T(0), wn = T(0);
 #pragma unroll
-        for (int m = 0; m < NV; ++m) dl = dl + sW[k * NV + m][l - 1] * W[k][m];
-#pragma unroll
-        for (int m = 0; m < NV; ++m) dr = dr + W[k][m] * sW[k * NV + m][l + 1];
+        for (int m = 0; m < NV; ++m) dot = dot + sW[k * NV + m][up] * W[k][m];
 #pragma unroll
         for (int m = 0; m < NV; ++m) wn = wn + W[k][m] * W[k][m];
         if (wn != T(0)) {
-          const T r = (S[k] > T(0)) ? dl / wn : dr / wn;
-          const T phi = philim3(sp.mthlim[k], r);
+          const T phi = philim3(sp.mthlim[k], dot / wn);
 #pragma unroll
           for (int m = 0; m < NV; ++m) W[k][m] = phi * W[k][m];
         }
@@ -567,16 +566,15 @@ __global__ void __launch_bounds__(SW_T) split3_kernel(Step3Args A) {
 #pragma unroll
       for (int k = 0; k < NW; ++k) {
         if (sp.mthlim[k] == 0) continue;
-        T dl = T(0), dr = T(0), wn = T(0);
+        // the ratio takes the neighbour on the upwind side
+        const int up = S[k] > T(0) ? l - 1 : l + 1;
+        T dot = T(0), wn = T(0);
 #pragma unroll
-        for (int m = 0; m < NV; ++m) dl = dl + sW[k * NV + m][l - 1] * W[k][m];
-#pragma unroll
-        for (int m = 0; m < NV; ++m) dr = dr + W[k][m] * sW[k * NV + m][l + 1];
+        for (int m = 0; m < NV; ++m) dot = dot + sW[k * NV + m][up] * W[k][m];
 #pragma unroll
         for (int m = 0; m < NV; ++m) wn = wn + W[k][m] * W[k][m];
         if (wn != T(0)) {
-          const T r = (S[k] > T(0)) ? dl / wn : dr / wn;
-          const T phi = philim3(sp.mthlim[k], r);
+          const T phi = philim3(sp.mthlim[k], dot / wn);
 #pragma unroll
           for (int m = 0; m < NV; ++m) W[k][m] = phi * W[k][m];
         }
