@@ -249,11 +249,8 @@ class Amr3Gpu : public AmrSolver {
     if (h_cfl) cudaFreeHost(h_cfl);
     if (d_mass) cudaFree(d_mass);
     for (cudaEvent_t e : {ev_a, ev_b, ev_run0, ev_run1}) if (e) cudaEventDestroy(e);
-    for (cudaEvent_t e : {sweep_ss.fork, sweep_ss.join[0], sweep_ss.join[1]}) if (e) cudaEventDestroy(e);
-    for (cudaStream_t x : sweep_ss.side) if (x) { cudaStreamSynchronize(x); cudaStreamDestroy(x); }
     if (st) cudaStreamDestroy(st);
   }
-  SweepStreams sweep_ss{};  // the side streams of the sweep directions
   void sync_stream() { AMR_CUDA(cudaStreamSynchronize(st)); stg.reset(); }
 
   int mitot(int m) const { return node[m].nx() + 2 * G3; }
@@ -1547,7 +1544,7 @@ class Amr3Gpu : public AmrSolver {
         const int sched = pick_schedule(lev, tt, ds != nullptr);
         a.queue = sched == 1 ? d_queue : nullptr;
         if (tt) AMR_CUDA(cudaEventRecord(ev_t0, st));
-        nkernels += launch_step3(a, L.items, L.faces, L.cells, st, f32, &sweep_ss);
+        nkernels += launch_step3(a, L.items, L.faces, L.cells, st, f32);
         if (tt) { AMR_CUDA(cudaEventRecord(ev_t1, st)); tune_pending = sched; }
       }
       if (timed) AMR_CUDA(cudaEventRecord(ev_b, st));
@@ -1586,7 +1583,7 @@ class Amr3Gpu : public AmrSolver {
           nkernels += launch_split3(b, it, st, f32);
         } else {
           for (int d = 0; d < 3; ++d) it[d] = L.comp0[(size_t)d * (np + 1) + k + 1] - L.comp0[(size_t)d * (np + 1) + k];
-          nkernels += launch_step3(b, it, L.face0[k + 1] - L.face0[k], L.cell0[k + 1] - L.cell0[k], st, f32, &sweep_ss);
+          nkernels += launch_step3(b, it, L.face0[k + 1] - L.face0[k], L.cell0[k + 1] - L.cell0[k], st, f32);
         }
         const long long f0 = L.fsv0[k], nf = L.fsv0[k + 1] - L.fsv0[k];
         if (nf > 0) {
@@ -2352,9 +2349,6 @@ class Amr3Gpu : public AmrSolver {
       lc.intratx[l] = intratx[l]; lc.intraty[l] = intraty[l]; lc.intratz[l] = intratz[l];
     }
     AMR_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    for (cudaStream_t& x : sweep_ss.side) AMR_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
-    AMR_CUDA(cudaEventCreateWithFlags(&sweep_ss.fork, cudaEventDisableTiming));
-    for (cudaEvent_t& e : sweep_ss.join) AMR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     retain_pool_memory();
     AllocStreamScope alloc_scope(st);
     for (cudaEvent_t* e : {&ev_a, &ev_b, &ev_run0, &ev_run1}) AMR_CUDA(cudaEventCreate(e));

@@ -39,6 +39,26 @@ __device__ __forceinline__ int find_patch(const long long* pre, int np, long lon
   return lo;
 }
 
+// The same for the lanes of a warp at consecutive places t0, t0+1, ... of the list (t clamped
+// to it by the caller): the warp searches for its first place 32 ways at a time, two dependent
+// reads for up to 1024 patches instead of ten, and a lane past that patch's end walks on.
+__device__ __forceinline__ int find_patch_warp(const long long* pre, int np, long long t) {
+  if (np == 1) return 0;
+  const int lane = threadIdx.x & 31;
+  const long long t0 = __shfl_sync(0xffffffffu, t, 0);
+  int lo = 0, n = np;  // the patch is one of lo .. lo+n-1
+  while (n > 1) {
+    const int step = (n + 31) / 32;
+    const int at = lo + lane * step;
+    const bool le = lane * step < n && pre[at] <= t0;
+    const int last = 31 - __clz(__ballot_sync(0xffffffffu, le) | 1u);
+    n = min(step, n - last * step);
+    lo += last * step;
+  }
+  while (lo + 1 < np && pre[lo + 1] <= t) ++lo;
+  return lo;
+}
+
 __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* p, double v) {
   atomicMax(p, (unsigned long long)__double_as_longlong(v));
 }
@@ -334,8 +354,8 @@ __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, 
   long long slot = 0;  // stash slot of pencil cell e (meaningful for e in 1..n1+1)
   PH ph;
   T W[NW][NV], S[NW], AM[NV], AP[NV];
+  const int pi = find_patch_warp(c0, A.np, g < first ? first : g < last ? g : last - 1);
   if (valid) {
-    const int pi = find_patch(c0, A.np, g);
     const PatchDev& P = A.patches[A.plist[pi]];
     const int mx = P.ihi - P.ilo + 1, my = P.jhi - P.jlo + 1, mz = P.khi - P.klo + 1;
     n1 = DIR == 1 ? mx : DIR == 2 ? my : mz;
@@ -638,8 +658,10 @@ __global__ void __launch_bounds__(128) face3_kernel(Step3Args A) {
   const long long first = A.face0[0], total = A.face0[A.np];
   constexpr int ss = STASH_BLK;
   const T* S = static_cast<const T*>(A.stash);
-  for (long long t = first + (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int pi = find_patch(A.face0, A.np, t);
+  for (long long w = first + (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); w < total; w += (long long)gridDim.x * blockDim.x) {
+    const long long t = w + (threadIdx.x & 31);
+    const int pi = find_patch_warp(A.face0, A.np, min(t, total - 1));
+    if (t >= total) break;
     const PatchDev& P = A.patches[A.plist[pi]];
     const int mx = P.ihi - P.ilo + 1, my = P.jhi - P.jlo + 1, mz = P.khi - P.klo + 1;
     // Thread t takes the face cells of its patch in brick order: slabs of FB_K k-planes,
@@ -781,12 +803,14 @@ __global__ void __launch_bounds__(256) update3_kernel(Step3Args A) {
   const long long fs = A.flux_stride;
   const double dt = A.dt_dev ? *A.dt_dev : A.dt;
   const T dtdx = (T)(dt / A.dx), dtdy = (T)(dt / A.dy), dtdz = (T)(dt / A.dz);
-  for (long long t = first + (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int pi = find_patch(A.cell0, A.np, t);
+  for (long long w = first + (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); w < total; w += (long long)gridDim.x * blockDim.x) {
+    const long long t = w + (threadIdx.x & 31);
+    const int pi = find_patch_warp(A.cell0, A.np, min(t, total - 1));
+    if (t >= total) break;
     const PatchDev& P = A.patches[A.plist[pi]];
     const int mx = P.ihi - P.ilo + 1, my = P.jhi - P.jlo + 1;
-    const long long loc = t - A.cell0[pi];
-    const int i = (int)(loc % mx) + 1, j = (int)((loc / mx) % my) + 1, k = (int)(loc / ((long long)mx * my)) + 1;
+    const unsigned loc = (unsigned)(t - A.cell0[pi]), row = loc / (unsigned)mx, lay = row / (unsigned)my;
+    const int i = (int)(loc - row * (unsigned)mx) + 1, j = (int)(row - lay * (unsigned)my) + 1, k = (int)lay + 1;
     const long long f0 = A.face0[pi];
     auto fidx = [&](int ii, int jj, int kk) { return f0 + ((long long)(kk - 1) * (my + 1) + (jj - 1)) * (mx + 1) + (ii - 1); };
     const long long plane = (long long)P.mitot * P.mjtot * P.mktot;
@@ -1415,36 +1439,22 @@ static void set_sweep_smem() {
   }();
   (void)done;
 }
-// the three sweep directions of a level, one launch each: x on s, y and z on the side
-// streams (if given) joined back before the face gather
+// the three sweep directions of a level, one launch each, after one another: y and z on
+// streams of their own beside x gained nothing any more (26.4 against 26.25 ms for 20 steps of
+// a 90^3 level, 19.9 against 19.6 ms for four coarse steps of a 48^3 three-level driver)
 template <class T, class PH>
-static int launch_sweeps(const Step3Args& a, const long long items[3], cudaStream_t s, const SweepStreams* ss) {
+static int launch_sweeps(const Step3Args& a, const long long items[3], cudaStream_t s) {
   auto tiles = [](long long n) { return (unsigned)((n + SW_OWN - 1) / SW_OWN); };
   constexpr int smem = sweep3_smem_bytes<T, PH>();
   set_sweep_smem<T, PH>();
   int n = 0;
-  cudaStream_t sy = s, sz = s;
-  if (ss) {
-    AMR_CUDA(cudaEventRecord(ss->fork, s));
-    AMR_CUDA(cudaStreamWaitEvent(ss->side[0], ss->fork, 0));
-    AMR_CUDA(cudaStreamWaitEvent(ss->side[1], ss->fork, 0));
-    sy = ss->side[0]; sz = ss->side[1];
-  }
   if (items[0] > 0) { sweep3_kernel<1, T, PH><<<tiles(items[0]), SW_T, smem, s>>>(a); ++n; }
-  if (items[1] > 0) { sweep3_kernel<2, T, PH><<<tiles(items[1]), SW_T, smem, sy>>>(a); ++n; }
-  if (items[2] > 0) { sweep3_kernel<3, T, PH><<<tiles(items[2]), SW_T, smem, sz>>>(a); ++n; }
-  if (ss) {
-    AMR_CUDA(cudaEventRecord(ss->join[0], ss->side[0]));
-    AMR_CUDA(cudaEventRecord(ss->join[1], ss->side[1]));
-    AMR_CUDA(cudaStreamWaitEvent(s, ss->join[0], 0));
-    AMR_CUDA(cudaStreamWaitEvent(s, ss->join[1], 0));
-  }
+  if (items[1] > 0) { sweep3_kernel<2, T, PH><<<tiles(items[1]), SW_T, smem, s>>>(a); ++n; }
+  if (items[2] > 0) { sweep3_kernel<3, T, PH><<<tiles(items[2]), SW_T, smem, s>>>(a); ++n; }
   return n;
 }
-
 template <class T, class PH>
-static int launch_step3_t(const Step3Args& a, const long long items[3], long long faces, long long cells, cudaStream_t s,
-                          const SweepStreams* ss) {
+static int launch_step3_t(const Step3Args& a, const long long items[3], long long faces, long long cells, cudaStream_t s) {
   auto tiles = [](long long n) { return (unsigned)((n + SW_OWN - 1) / SW_OWN); };
   constexpr int smem = sweep3_smem_bytes<T, PH>();
   int n = 0;
@@ -1469,7 +1479,7 @@ static int launch_step3_t(const Step3Args& a, const long long items[3], long lon
       ++n;
     }
   } else {
-    n += launch_sweeps<T, PH>(a, items, s, ss);
+    n += launch_sweeps<T, PH>(a, items, s);
   }
   AMR_CUDA(cudaGetLastError());
   if (faces > 0) { face3_kernel<T, PH::NV><<<grid_for(faces, 128), 128, 0, s>>>(a); ++n; }
@@ -1496,14 +1506,13 @@ int launch_split3(const Step3Args& a, const long long items[3], cudaStream_t s, 
   return launch_split3_t<double, Euler3Phys<double>>(a, items, s);
 }
 
-int launch_step3(const Step3Args& a, const long long items[3], long long faces, long long cells, cudaStream_t s, bool f32,
-                 const SweepStreams* ss) {
+int launch_step3(const Step3Args& a, const long long items[3], long long faces, long long cells, cudaStream_t s, bool f32) {
   if (a.sp.solver == SOLVER3_SWIRL) {
-    if (f32) return launch_step3_t<float, Swirl3Phys<float>>(a, items, faces, cells, s, ss);
-    return launch_step3_t<double, Swirl3Phys<double>>(a, items, faces, cells, s, ss);
+    if (f32) return launch_step3_t<float, Swirl3Phys<float>>(a, items, faces, cells, s);
+    return launch_step3_t<double, Swirl3Phys<double>>(a, items, faces, cells, s);
   }
-  if (f32) return launch_step3_t<float, Euler3Phys<float>>(a, items, faces, cells, s, ss);
-  return launch_step3_t<double, Euler3Phys<double>>(a, items, faces, cells, s, ss);
+  if (f32) return launch_step3_t<float, Euler3Phys<float>>(a, items, faces, cells, s);
+  return launch_step3_t<double, Euler3Phys<double>>(a, items, faces, cells, s);
 }
 
 void launch_expand_fadqad3(const int* plist, const long long* pre, int np, const PatchDev* patches, int rx, int ry, int rz,

@@ -114,15 +114,7 @@ struct Gauge3Job { int patch; int ii, jj, kk; int slot; double xoff, yoff, zoff;
 // flux differencing; FP64 registers, register corrections, averages and totals).
 // interfaces_per_dir: the interfaces (comp0 ranges) of each sweep direction.
 // returns the number of kernels launched
-// Two side streams and the events that fork them off the solve's stream and join them back:
-// the three sweep directions of a level (independent of one another) then run at once, and
-// the tail blocks of one direction overlap the others instead of leaving SMs idle.
-struct SweepStreams {
-  cudaStream_t side[2];
-  cudaEvent_t fork, join[2];
-};
-int launch_step3(const Step3Args& a, const long long interfaces_per_dir[3], long long faces, long long cells, cudaStream_t s, bool f32,
-                 const SweepStreams* ss = nullptr);
+int launch_step3(const Step3Args& a, const long long interfaces_per_dir[3], long long faces, long long cells, cudaStream_t s, bool f32);
 // the Godunov-split step of the level (stepgrid_dimSplit.f): x, y and z sweeps with their
 // updates, interfaces_per_dir counting the split pencils (scomp0); returns launches made
 int launch_split3(const Step3Args& a, const long long interfaces_per_dir[3], cudaStream_t s, bool f32);
