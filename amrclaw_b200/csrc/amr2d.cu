@@ -2880,13 +2880,15 @@ class Amr2Gpu {
     std::vector<long long> off(1, 0);
     for (int lev = 1; lev <= lfine; ++lev)
       for (int m : lgrids[lev]) { pl.push_back(m); off.push_back(off.back() + (long long)nvar * node[m].nx() * node[m].ny()); }
+    long long most = 0;
+    for (int m : pl) most = std::max(most, (long long)node[m].nx() * node[m].ny());
     const long long tot = off.back();
     off.pop_back();
     if (tot == 0) return;
     DBuf<double> d; d.ensure(tot);
     DBuf<int> dp; dp.upload(pl, st, stg);
     DBuf<long long> doff; doff.upload(off, st, stg);
-    launch_gather_interior2(pool.d, d_patches.d, dp.d, doff.d, (int)pl.size(), nvar, d.d, st, f32);
+    launch_gather_interior2(pool.d, d_patches.d, dp.d, doff.d, (int)pl.size(), most, nvar, d.d, st, f32);
     AMR_CUDA(cudaMemcpyAsync(out, d.d, sizeof(double) * tot, cudaMemcpyDeviceToHost, st));
     sync_stream();
     d.free(); dp.free(); doff.free();
@@ -2910,7 +2912,9 @@ void Amr2Gpu::output(double t) {
   for (int lev = 1; lev <= lfine; ++lev) {
     ensure(lev, NEED_STEP);
     if (binary) continue;
-    launch_zero_tiny(pool.d, d_patches.d, plan[lev].d_plist.d, (int)plan[lev].plist.size(), nvar, st, f32);
+    long long most = 0;
+    for (int m : plan[lev].plist) most = std::max(most, (long long)node[m].nx() * node[m].ny());
+    launch_zero_tiny(pool.d, d_patches.d, plan[lev].d_plist.d, (int)plan[lev].plist.size(), most, nvar, st, f32);
     ++nkernels;
   }
   if (write_output && binary) {

@@ -2808,10 +2808,12 @@ class Amr3Gpu : public AmrSolver {
     for (int lev = 1; lev <= lfine; ++lev) {
       ensure(lev, NEED_STEP);
       if (binary) continue;  // the binary form zeroes nothing
-      launch_zero_tiny3(pool.d, d_patches.d, plan[lev].d_plist.d, (int)plan[lev].plist.size(), nvar, st, f32);
+      long long most = 0;
+      for (int m : plan[lev].plist) most = std::max(most, (long long)node[m].nx() * node[m].ny() * node[m].nz());
+      launch_zero_tiny3(pool.d, d_patches.d, plan[lev].d_plist.d, (int)plan[lev].plist.size(), most, nvar, st, f32);
       ++nkernels;
       if (aux) {
-        launch_zero_tiny3(pool.d, d_patches.d, plan[lev].d_plist.d, (int)plan[lev].plist.size(), p.naux, st, f32, true);
+        launch_zero_tiny3(pool.d, d_patches.d, plan[lev].d_plist.d, (int)plan[lev].plist.size(), most, p.naux, st, f32, true);
         ++nkernels;
       }
     }

@@ -185,14 +185,16 @@ void launch_flags2(const void* pool, const PatchDev* patches, const int* plist, 
                    int use_old, int flag_component, double tolsp, int nvar, int8_t* out, cudaStream_t s, bool f32);
 void launch_gauges2(const void* pool, const PatchDev* patches, const GaugeJob* jobs, int njobs, int nvar,
                     double* out, cudaStream_t s, bool f32);
-void launch_zero_tiny(void* pool, const PatchDev* patches, const int* plist, int np, int nvar, cudaStream_t s, bool f32);
+// max_cells: interior cells of the largest listed patch (sizes the launch; here and below)
+void launch_zero_tiny(void* pool, const PatchDev* patches, const int* plist, int np, long long max_cells, int nvar, cudaStream_t s,
+                      bool f32);
 void launch_mass2(const void* pool, const PatchDev* patches, const int* plist, int np, double* out, cudaStream_t s, bool f32,
                   int mcapa = 0);
 // whole arrays (ghost cells included) in the reference's q(m,i,j) order, for binary output
 void launch_gather_enlarged2(const void* pool, const PatchDev* patches, const int* plist, const long long* outoff, int np,
                              int nvar, double* out, int split, cudaStream_t s, bool f32);
 void launch_gather_interior2(const void* pool, const PatchDev* patches, const int* plist, const long long* outoff,
-                             int np, int nvar, double* out, cudaStream_t s, bool f32);
+                             int np, long long max_cells, int nvar, double* out, cudaStream_t s, bool f32);
 size_t step2_smem_bytes(int solver, bool f32);
 // Richardson estimation (errest.f): rect_of[k] is the scratch rect of virtual patch k
 void launch_coarsen2(void* pool, const ScratchRect* rects, const int* rect_of, const PatchDev* vp, int np, int nvar,

@@ -146,8 +146,9 @@ struct Setaux3Job { long long aux, f0; int mi, mj, mk, pad; };
 void launch_setaux3(void* pool, const Setaux3Job* jobs, int njobs, long long max_cells, const double* fac, int copies,
                     cudaStream_t s, bool f32);
 // valout.f90:140-147: |q| < 1e-90 of the interior cells of plist set to 0 in place
-void launch_zero_tiny3(void* pool, const PatchDev* patches, const int* plist, int np, int nvar, cudaStream_t s, bool f32,
-                       bool aux = false);
+// (max_cells: interior cells of the largest listed patch)
+void launch_zero_tiny3(void* pool, const PatchDev* patches, const int* plist, int np, long long max_cells, int nvar, cudaStream_t s,
+                       bool f32, bool aux = false);
 // b4step3 of the time-modulated swirl: aux = c * aux0 over the enlarged patches of plist
 // (max_cells: the largest enlarged patch)
 void launch_b4step3(void* pool, const PatchDev* patches, const int* plist, int np, int naux, long long max_cells, double c,
