@@ -2363,6 +2363,7 @@ class Amr3Gpu : public AmrSolver {
     AMR_CUDA(cudaMalloc(&d_queue, sizeof(unsigned int)));
     AMR_CUDA(cudaEventCreate(&ev_t0)); AMR_CUDA(cudaEventCreate(&ev_t1));
     AMR_CUDA(cudaMallocHost((void**)&h_sub, sizeof(Substep3) * 12));
+    stg.soon = (size_t)32 << 20;
     {
       // sweep staging and face fluxes: reserved at once for twice a level-1 sweep
       const long long n = (long long)nxc * nyc * nzc;

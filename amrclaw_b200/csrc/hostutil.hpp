@@ -202,34 +202,41 @@ inline void set_arena_limits(Arena& pool, Arena& regs, long long bytes) {
 // queued without the driver's pageable bounce. Space is reused only after the
 // stream has been synchronized (Staging::reset is called right after each sync).
 //
-// The memory is a chain of chunks that grows by as much as it holds: pinning costs about
-// 0.3 ms per MB, and most solves stage a few MB between two synchronisations. (One ring of
-// 256 MB pinned at start-up cost a 3D solve about 130 ms of its own.) A chunk is kept until
-// the context ends, so growing neither frees nor waits; past LIMIT bytes in all, the stream
-// is synchronized and the chain starts over instead.
+// The memory is a chain of chunks: pinning costs about 0.3 ms per MB, and most solves stage
+// a few MB between two synchronisations. (One ring of 256 MB pinned at start-up cost a 3D
+// solve about 130 ms of its own.) The chain grows by what it holds up to `soon`; then it
+// synchronizes the stream and starts over when it is full, and grows again, up to LIMIT, each
+// time that has happened WRAPS times. A chunk is kept until the context ends, so growing
+// neither frees nor waits.
 struct Staging {
   struct Chunk { char* h; size_t cap; };
-  static constexpr size_t FIRST = (size_t)4 << 20, LIMIT = (size_t)256 << 20;
+  static constexpr size_t FIRST = (size_t)1 << 20, LIMIT = (size_t)256 << 20;
+  static constexpr int WRAPS = 8;
   std::vector<Chunk> chunks;
   size_t at = 0, used = 0, held = 0;  // chunk in use, bytes used of it, bytes of all chunks
+  int wraps = 0;                      // since the chain last grew
+  size_t soon = (size_t)8 << 20;      // grown to at once (3D stages more between synchronisations)
+  void seek(size_t n2) {
+    while (at < chunks.size() && used + n2 > chunks[at].cap) { ++at; used = 0; }
+  }
   const void* put(const void* src, size_t n, cudaStream_t s) {
     const size_t n2 = (n + 255) & ~(size_t)255;
-    while (at < chunks.size() && used + n2 > chunks[at].cap) { ++at; used = 0; }
+    seek(n2);
+    if (at == chunks.size() && held >= soon && (wraps < WRAPS || held >= LIMIT)) {
+      ++g_stage_wraps;
+      ++wraps;
+      AMR_CUDA(cudaStreamSynchronize(s));
+      reset();
+      seek(n2);
+    }
     if (at == chunks.size()) {
-      if (held >= LIMIT) {
-        ++g_stage_wraps;
-        AMR_CUDA(cudaStreamSynchronize(s));
-        reset();
-        while (at < chunks.size() && n2 > chunks[at].cap) ++at;
-      }
-      if (at == chunks.size()) {
-        const size_t cap = std::max<size_t>({n2, std::min(held, LIMIT - std::min(held, LIMIT)), FIRST});
-        char* h = nullptr;
-        AMR_CUDA(cudaMallocHost((void**)&h, cap));
-        chunks.push_back(Chunk{h, cap});
-        held += cap;
-        used = 0;
-      }
+      const size_t cap = std::max<size_t>({n2, std::min(held, LIMIT - std::min(held, LIMIT)), FIRST});
+      char* h = nullptr;
+      AMR_CUDA(cudaMallocHost((void**)&h, cap));
+      chunks.push_back(Chunk{h, cap});
+      held += cap;
+      used = 0;
+      wraps = 0;
     }
     char* dst = chunks[at].h + used;
     const auto t0 = std::chrono::steady_clock::now();
@@ -244,6 +251,7 @@ struct Staging {
     for (const Chunk& c : chunks) cudaFreeHost(c.h);
     chunks.clear();
     at = used = held = 0;
+    wraps = 0;
   }
 };
 
