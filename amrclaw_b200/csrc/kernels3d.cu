@@ -476,6 +476,18 @@ __global__ void __launch_bounds__(SW_T, sweep_min_blocks<T>()) sweep3_kernel(Ste
   sweep3_tile<DIR, T, PH>(A, blockIdx.x, reinterpret_cast<T (*)[SW_T]>(sweep_smem));
 }
 
+// all three directions in one launch: the first nx blocks take the x tiles, the next the y
+// tiles (to nxy), the rest the z tiles
+template <class T, class PH>
+__global__ void __launch_bounds__(SW_T, sweep_min_blocks<T>()) sweep3_all_kernel(Step3Args A, unsigned nx, unsigned nxy) {
+  extern __shared__ __align__(16) unsigned char sweep_smem[];
+  T (*sW)[SW_T] = reinterpret_cast<T (*)[SW_T]>(sweep_smem);
+  const unsigned b = blockIdx.x;
+  if (b < nx) sweep3_tile<1, T, PH>(A, b, sW);
+  else if (b < nxy) sweep3_tile<2, T, PH>(A, b - nx, sW);
+  else sweep3_tile<3, T, PH>(A, b - nxy, sW);
+}
+
 // persistent work queue over the tiles of all three directions of the level (x tiles,
 // then y, then z): resident blocks take the next tile from an atomic counter until none
 // is left. The tiles are independent (each writes its own stash slots), so no block
@@ -1435,19 +1447,33 @@ static void set_sweep_smem() {
     AMR_CUDA(cudaFuncSetAttribute(sweep3_kernel<1, T, PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     AMR_CUDA(cudaFuncSetAttribute(sweep3_kernel<2, T, PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     AMR_CUDA(cudaFuncSetAttribute(sweep3_kernel<3, T, PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    AMR_CUDA(cudaFuncSetAttribute(sweep3_all_kernel<T, PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     return true;
   }();
   (void)done;
 }
-// the three sweep directions of a level, one launch each, after one another: y and z on
-// streams of their own beside x gained nothing any more (26.4 against 26.25 ms for 20 steps of
-// a 90^3 level, 19.9 against 19.6 ms for four coarse steps of a 48^3 three-level driver)
+// Tiles up to which the three directions go in one launch: nine quarters of the blocks that
+// are resident at once (148 SMs). A level below that leaves SMs idle in launches of its own,
+// one direction after another; above it the last wave matters less than that a kernel of one
+// direction has a third of the code (and FP64 fewer spills). 10 steps of a uniform level with
+// the frame read back, one launch against three: FP64 16^3 846 / 1129 us, 32^3 (972 tiles)
+// 1495 / 1526, 36^3 (1353) 2105 / 2031, 48^3 3146 / 2964; FP32 16^3 825 / 951, 36^3 1176 /
+// 1282, 48^3 (3063) 2147 / 2004. (Streams of their own for y and z, joined before the gather:
+// 16^3 987 us, and nothing gained from 48^3 on.)
+template <class T>
+constexpr unsigned merge_tiles() { return 148u * (unsigned)sweep_min_blocks<T>() * 9u / 4u; }
+// the three sweep directions of a level, in one launch or one each
 template <class T, class PH>
 static int launch_sweeps(const Step3Args& a, const long long items[3], cudaStream_t s) {
   auto tiles = [](long long n) { return (unsigned)((n + SW_OWN - 1) / SW_OWN); };
   constexpr int smem = sweep3_smem_bytes<T, PH>();
   set_sweep_smem<T, PH>();
   int n = 0;
+  const unsigned nx = tiles(items[0]), nxy = nx + tiles(items[1]), nall = nxy + tiles(items[2]);
+  if (nall <= merge_tiles<T>()) {
+    if (nall > 0) { sweep3_all_kernel<T, PH><<<nall, SW_T, smem, s>>>(a, nx, nxy); ++n; }
+    return n;
+  }
   if (items[0] > 0) { sweep3_kernel<1, T, PH><<<tiles(items[0]), SW_T, smem, s>>>(a); ++n; }
   if (items[1] > 0) { sweep3_kernel<2, T, PH><<<tiles(items[1]), SW_T, smem, s>>>(a); ++n; }
   if (items[2] > 0) { sweep3_kernel<3, T, PH><<<tiles(items[2]), SW_T, smem, s>>>(a); ++n; }
