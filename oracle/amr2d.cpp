@@ -708,12 +708,17 @@ struct Amr2 {
     FArr val{valp, nvar, nrow, ncol};
     const double hxmarg = hx * 0.01, hymarg = hy * 0.01;
     if (xperdom && (yperdom || spheredom)) return;
+    // A periodic piece (prefilrecur) may lie wholly beyond a wall or extrapolation face: a
+    // source outside its array is not read, and the patch's own call sets the cell later.
+    auto cp = [&](int m, int i, int j, int si, int sj) {
+      if (si >= 1 && si <= nrow && sj >= 1 && sj <= ncol) val(m, i, j) = val(m, si, sj);
+    };
     if (xlo_p < xlower - hxmarg) {
       int nxl = (int)((xlower + hxmarg - xlo_p) / hx);
       if (mthbc[1] == 1) {
-        for (int j = 1; j <= ncol; ++j) for (int i = 1; i <= nxl; ++i) for (int m = 1; m <= nvar; ++m) val(m, i, j) = val(m, nxl + 1, j);
+        for (int j = 1; j <= ncol; ++j) for (int i = 1; i <= nxl; ++i) for (int m = 1; m <= nvar; ++m) cp(m, i, j, nxl + 1, j);
       } else if (mthbc[1] == 3) {
-        for (int j = 1; j <= ncol; ++j) for (int i = 1; i <= nxl; ++i) for (int m = 1; m <= nvar; ++m) val(m, i, j) = val(m, 2 * nxl + 1 - i, j);
+        for (int j = 1; j <= ncol; ++j) for (int i = 1; i <= nxl; ++i) for (int m = 1; m <= nvar; ++m) cp(m, i, j, 2 * nxl + 1 - i, j);
         for (int j = 1; j <= ncol; ++j) for (int i = 1; i <= nxl; ++i) val(2, i, j) = -val(2, i, j);
       } else if (mthbc[1] == 0) throw std::runtime_error("user BC not provided");
     }
@@ -721,18 +726,18 @@ struct Amr2 {
       int nxr = (int)((xhi_p - xupper + hxmarg) / hx);
       int ibeg = std::max(nrow - nxr + 1, 1);
       if (mthbc[2] == 1) {
-        for (int i = ibeg; i <= nrow; ++i) for (int j = 1; j <= ncol; ++j) for (int m = 1; m <= nvar; ++m) val(m, i, j) = val(m, ibeg - 1, j);
+        for (int i = ibeg; i <= nrow; ++i) for (int j = 1; j <= ncol; ++j) for (int m = 1; m <= nvar; ++m) cp(m, i, j, ibeg - 1, j);
       } else if (mthbc[2] == 3) {
-        for (int i = ibeg; i <= nrow; ++i) for (int j = 1; j <= ncol; ++j) for (int m = 1; m <= nvar; ++m) val(m, i, j) = val(m, 2 * ibeg - 1 - i, j);
+        for (int i = ibeg; i <= nrow; ++i) for (int j = 1; j <= ncol; ++j) for (int m = 1; m <= nvar; ++m) cp(m, i, j, 2 * ibeg - 1 - i, j);
         for (int i = ibeg; i <= nrow; ++i) for (int j = 1; j <= ncol; ++j) val(2, i, j) = -val(2, i, j);
       } else if (mthbc[2] == 0) throw std::runtime_error("user BC not provided");
     }
     if (ylo_p < ylower - hymarg) {
       int nyb = (int)((ylower + hymarg - ylo_p) / hy);
       if (mthbc[3] == 1) {
-        for (int j = 1; j <= nyb; ++j) for (int i = 1; i <= nrow; ++i) for (int m = 1; m <= nvar; ++m) val(m, i, j) = val(m, i, nyb + 1);
+        for (int j = 1; j <= nyb; ++j) for (int i = 1; i <= nrow; ++i) for (int m = 1; m <= nvar; ++m) cp(m, i, j, i, nyb + 1);
       } else if (mthbc[3] == 3) {
-        for (int j = 1; j <= nyb; ++j) for (int i = 1; i <= nrow; ++i) for (int m = 1; m <= nvar; ++m) val(m, i, j) = val(m, i, 2 * nyb + 1 - j);
+        for (int j = 1; j <= nyb; ++j) for (int i = 1; i <= nrow; ++i) for (int m = 1; m <= nvar; ++m) cp(m, i, j, i, 2 * nyb + 1 - j);
         for (int j = 1; j <= nyb; ++j) for (int i = 1; i <= nrow; ++i) val(3, i, j) = -val(3, i, j);
       } else if (mthbc[3] == 0) throw std::runtime_error("user BC not provided");
     }
@@ -740,9 +745,9 @@ struct Amr2 {
       int nyt = (int)((yhi_p - yupper + hymarg) / hy);
       int jbeg = std::max(ncol - nyt + 1, 1);
       if (mthbc[4] == 1) {
-        for (int j = jbeg; j <= ncol; ++j) for (int i = 1; i <= nrow; ++i) for (int m = 1; m <= nvar; ++m) val(m, i, j) = val(m, i, jbeg - 1);
+        for (int j = jbeg; j <= ncol; ++j) for (int i = 1; i <= nrow; ++i) for (int m = 1; m <= nvar; ++m) cp(m, i, j, i, jbeg - 1);
       } else if (mthbc[4] == 3) {
-        for (int j = jbeg; j <= ncol; ++j) for (int i = 1; i <= nrow; ++i) for (int m = 1; m <= nvar; ++m) val(m, i, j) = val(m, i, 2 * jbeg - 1 - j);
+        for (int j = jbeg; j <= ncol; ++j) for (int i = 1; i <= nrow; ++i) for (int m = 1; m <= nvar; ++m) cp(m, i, j, i, 2 * jbeg - 1 - j);
         for (int j = jbeg; j <= ncol; ++j) for (int i = 1; i <= nrow; ++i) val(3, i, j) = -val(3, i, j);
       } else if (mthbc[4] == 0) throw std::runtime_error("user BC not provided");
     }
