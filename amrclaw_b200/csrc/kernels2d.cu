@@ -1001,6 +1001,8 @@ __device__ __forceinline__ void bc_op(const BcArgs& a, int op, int phase, int nb
   const long long plane = (long long)nrow * ncol;
   auto V = [&](int m, int i, int j) -> T& { return v[m * plane + (long long)(j - 1) * nrow + (i - 1)]; };
   const int nvar = a.nvar;
+  // A periodic piece may lie wholly beyond a wall or extrapolation face and hold no interior
+  // cell: a source outside the array is not read, and the cell is set later with its patch's ghosts.
   if (phase == 0) {
     const int nl = (o.nxl > 0 && (o.bxl == 1 || o.bxl == 3)) ? o.nxl : 0;
     const int nr = (o.ibeg > 0 && (o.bxr == 1 || o.bxr == 3)) ? nrow - o.ibeg + 1 : 0;
@@ -1010,11 +1012,13 @@ __device__ __forceinline__ void bc_op(const BcArgs& a, int op, int phase, int nb
       if (k < nl) {
         const int i = k + 1;
         const int src = (o.bxl == 1) ? o.nxl + 1 : 2 * o.nxl + 1 - i;
+        if (src < 1 || src > nrow) continue;
         for (int m = 0; m < nvar; ++m) V(m, i, j) = V(m, src, j);
         if (o.bxl == 3) V(1, i, j) = -V(1, i, j);
       } else {
         const int i = o.ibeg + (k - nl);
         const int src = (o.bxr == 1) ? o.ibeg - 1 : 2 * o.ibeg - 1 - i;
+        if (src < 1 || src > nrow) continue;
         for (int m = 0; m < nvar; ++m) V(m, i, j) = V(m, src, j);
         if (o.bxr == 3) V(1, i, j) = -V(1, i, j);
       }
@@ -1028,11 +1032,13 @@ __device__ __forceinline__ void bc_op(const BcArgs& a, int op, int phase, int nb
       if (k < nb) {
         const int j = k + 1;
         const int src = (o.byl == 1) ? o.nyb + 1 : 2 * o.nyb + 1 - j;
+        if (src < 1 || src > ncol) continue;
         for (int m = 0; m < nvar; ++m) V(m, i, j) = V(m, i, src);
         if (o.byl == 3) V(2, i, j) = -V(2, i, j);
       } else {
         const int j = o.jbeg + (k - nb);
         const int src = (o.byr == 1) ? o.jbeg - 1 : 2 * o.jbeg - 1 - j;
+        if (src < 1 || src > ncol) continue;
         for (int m = 0; m < nvar; ++m) V(m, i, j) = V(m, i, src);
         if (o.byr == 3) V(2, i, j) = -V(2, i, j);
       }
