@@ -74,13 +74,14 @@ def workload(name: str):
 
 
 # FP64 operations per cell-update of the 3D Euler CTU (transverse_waves 22) step kernels:
-# dadd + dmul + 2*dfma thread instructions of the three sweeps of a level-1 step, divided by
-# its cells (ncu instruction counts; the count does not depend on the patch sizes)
-FLOPS_PER_CELL_UPDATE_3D = 10.4e3
+# dadd + dmul + 2*dfma thread instructions of the three sweeps of a step of a 90^3 level
+# whose tiles are all subsonic, divided by its cells (ncu instruction counts; supersonic
+# tiles do about 10.4e3)
+FLOPS_PER_CELL_UPDATE_3D = 8.18e3
 # DRAM bytes per cell-update of the same kernels (sweeps, face gather, update): ncu
-# dram__bytes_read.sum + dram__bytes_write.sum of a level-1 substep of the 64^3 blast,
-# 1,070 MB over 262,144 cell-updates
-DRAM_BYTES_PER_CELL_UPDATE_3D = 1070.2e6 / 262144
+# dram__bytes_read.sum + dram__bytes_write.sum of a step of a 90^3 level, 3,143 MB over
+# 729,000 cell-updates
+DRAM_BYTES_PER_CELL_UPDATE_3D = 3143.0e6 / 729000
 
 
 def fp64_peak_tflops() -> float:
@@ -564,7 +565,7 @@ def main():
                      "traffic": (DRAM_BYTES_PER_CELL_UPDATE_3D * kern_cells / step_launches
                                  if headline and step_launches else None),
                      "traffic_note": "DRAM bytes per level substep of the step kernels: ncu bytes per cell-update "
-                                     "of a level-1 substep times the average cells of a timed substep",
+                                     "of a 90^3 level times the average cells of a timed substep",
                      "kernel": "sweep3<1..3> + face3 + update3" if ndim == 3 else "step2 sweeps + update",
                      "peak_kind": peak_kind,
                      "bytes_per_cell_update": bytes_per_update,
