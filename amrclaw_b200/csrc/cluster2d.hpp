@@ -1,5 +1,5 @@
 // Host-side integer algorithms of 2D regridding: flag buffering and projection,
-// proper-nesting masks, point collation and Berger-Rigoutsos bisection.
+// proper-nesting masks, point collation and the cut of a Berger-Rigoutsos bisection.
 //
 // These consume the per-cell gradient flags computed on the device and produce
 // the new patch rectangles. Each function follows the reference algorithm named
@@ -9,8 +9,7 @@
 //   nesting masks     src/2d/setdomflags.f:22-207, griddomshrink.f:24-82,
 //                     griddomup.f:16-116, setPhysBndryFlags.f:28-78
 //   sort_unique       src/2d/drivesort.f:7-62 with quick_sort1.f:22-167
-//   bisect            src/2d/smartbis.f:25-177, signs.f:16-71, findcut.f:7-130,
-//                     moment.f:16-75
+//   find_cut_sig      src/2d/findcut.f:7-130
 //   nest_check        src/2d/nestck2.f:37-176, baseCheck.f:19-240
 #pragma once
 #include <algorithm>
@@ -107,55 +106,9 @@ inline void sort_unique(std::vector<Pt>& pts, int isize, int mbuff) {
   pts.swap(out);
 }
 
-// Bounding box and fill ratio of a cluster of points (moment.f).
-inline double bbox_usage(const Pt* p, int n, int rect[4]) {
-  int i0 = p[0].i, i1 = p[0].i, j0 = p[0].j, j1 = p[0].j;
-  for (int k = 0; k < n; ++k) {
-    i0 = std::min(i0, p[k].i); i1 = std::max(i1, p[k].i);
-    j0 = std::min(j0, p[k].j); j1 = std::max(j1, p[k].j);
-  }
-  rect[0] = i0; rect[1] = i1; rect[2] = j0; rect[3] = j1;
-  return (double)n / (double)((i1 - i0 + 1) * (j1 - j0 + 1));
-}
-
-// Best cut of a cluster from its row/column signatures (signs.f + findcut.f).
-// Returns the 1-based cut index (0: no acceptable cut) and the direction (1: x, 2: y).
-inline int find_cut(const Pt* p, int n, int idim, int jdim, int& dir) {
-  std::vector<int> is(idim + 2, 0), js(jdim + 2, 0);
-  for (int k = 0; k < n; ++k) { is[p[k].i + 1] += 1; js[p[k].j + 1] += 1; }
-  int ilo = 1, ihi = idim, jlo = 1, jhi = jdim;
-  for (int t = 1; t <= idim; ++t) if (is[t] != 0) { ilo = t; break; }
-  for (int t = 1; t <= idim; ++t) if (is[idim + 1 - t] != 0) { ihi = idim + 1 - t; break; }
-  for (int t = 1; t <= jdim; ++t) if (js[t] != 0) { jlo = t; break; }
-  for (int t = 1; t <= jdim; ++t) if (js[jdim + 1 - t] != 0) { jhi = jdim + 1 - t; break; }
-  for (int i = ilo; i <= ihi; ++i) if (is[i] == 0) { dir = 1; return i; }
-  for (int j = jlo; j <= jhi; ++j) if (js[j] == 0) { dir = 2; return j; }
-  auto lap = [](std::vector<int>& s, int lo, int hi, int& best, int& idx) {
-    int pre = s[lo];
-    for (int i = lo + 1; i <= hi - 1; ++i) { const int cur = s[i]; s[i] = s[i + 1] - 2 * cur + pre; pre = cur; }
-    best = 0; idx = 0;
-    const int mid = (lo + hi) / 2;
-    for (int i = lo + 2; i <= hi - 2 + 1; ++i) {
-      const int a = s[i - 1], b = s[i], d = std::abs(a - b);
-      if (a * b < 0) {
-        if (d > best) { best = d; idx = i; }
-        else if (d == best && std::abs(i - mid) < std::abs(idx - mid)) idx = i;
-      }
-    }
-  };
-  int bi, ii, bj, ij;
-  lap(is, ilo, ihi, bi, ii);
-  lap(js, jlo, jhi, bj, ij);
-  int index, best;
-  if (bi > bj) { index = ii; dir = 1; best = bi; }
-  else if (bi < bj) { index = ij; dir = 2; best = bj; }
-  else if (std::abs(ii - (ilo + ihi) / 2) < std::abs(ij - (jlo + jhi) / 2)) { index = ii; dir = 1; best = bi; }
-  else { index = ij; dir = 2; best = bj; }
-  if (best < 2) index = 0;
-  return index;
-}
-
-// find_cut on signatures already counted (is, js: counts at 1-based positions 1..idim, 1..jdim).
+// Best cut of a cluster from its row/column signatures (findcut.f; is, js: counts at 1-based
+// positions 1..idim, 1..jdim). Returns the 1-based cut index (0: no acceptable cut) and the
+// direction (1: x, 2: y).
 inline int find_cut_sig(std::vector<int> is, std::vector<int> js, int idim, int jdim, int& dir) {
   int ilo = 1, ihi = idim, jlo = 1, jhi = jdim;
   for (int t = 1; t <= idim; ++t) if (is[t] != 0) { ilo = t; break; }
@@ -187,43 +140,6 @@ inline int find_cut_sig(std::vector<int> is, std::vector<int> js, int idim, int 
   else { index = ij; dir = 2; best = bj; }
   if (best < 2) index = 0;
   return index;
-}
-
-// Partition pts[a..b] (inclusive) so that points with coordinate >= cut stay at the
-// front, in the in-place swap order of smartbis.f:128-154. Returns the count at the front.
-inline int split_front(std::vector<Pt>& pts, int a, int b, int dir, int cut) {
-  int top = a - 1, bot = b + 1, i = a;
-  auto c = [&](int k) { return dir == 1 ? pts[k].i + 1 : pts[k].j + 1; };  // 1-based coordinate
-  while (true) {
-    if (c(i) < cut) {
-      --bot;
-      std::swap(pts[bot], pts[i]);
-      if (top + 1 < bot) continue;
-      break;
-    }
-    ++top;
-    if (top + 1 >= bot) break;
-    ++i;
-  }
-  return top - a + 1;
-}
-
-// Berger-Rigoutsos bisection of a sorted point list into clusters (smartbis.f).
-inline void bisect(std::vector<Pt>& pts, double cutoff, int idim, int jdim, std::vector<int>& cnt) {
-  cnt.assign(1, (int)pts.size());
-  int icl = 0, ist = 0;
-  while (icl < (int)cnt.size()) {
-    const int n = cnt[icl];
-    int rect[4];
-    const double use = bbox_usage(&pts[ist], n, rect);
-    if (use >= cutoff) { ist += n; ++icl; continue; }
-    int dir = 0;
-    const int cut = find_cut(&pts[ist], n, idim, jdim, dir);
-    if (cut == 0) { ist += n; ++icl; continue; }
-    const int front = split_front(pts, ist, ist + n - 1, dir, cut);
-    cnt[icl] = front;
-    cnt.insert(cnt.begin() + icl + 1, n - front);
-  }
 }
 
 }  // namespace amrb
