@@ -2046,7 +2046,7 @@ class Amr3Gpu : public AmrSolver {
       locmax = 0; idx = 0; mid = (l0 + h0) / 2;
       for (int t = l0 + 2; t <= h0 - 2 + 1; ++t) {
         const int t1 = sc[t - 1], t2 = sc[t], dd = std::abs(t1 - t2);
-        if (t1 * t2 < 0) {
+        if ((t1 < 0 && t2 > 0) || (t1 > 0 && t2 < 0)) {  // (a product of two counts can pass 32 bits)
           if (dd > locmax) { locmax = dd; idx = t; }
           else if (dd == locmax && std::abs(t - mid) < std::abs(idx - mid)) idx = t;
         }

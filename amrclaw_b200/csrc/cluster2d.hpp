@@ -124,7 +124,7 @@ inline int find_cut_sig(std::vector<int> is, std::vector<int> js, int idim, int 
     const int mid = (lo + hi) / 2;
     for (int i = lo + 2; i <= hi - 2 + 1; ++i) {
       const int a = s[i - 1], b = s[i], d = std::abs(a - b);
-      if (a * b < 0) {
+      if ((a < 0 && b > 0) || (a > 0 && b < 0)) {  // (a product of two counts can pass 32 bits)
         if (d > best) { best = d; idx = i; }
         else if (d == best && std::abs(i - mid) < std::abs(idx - mid)) idx = i;
       }

@@ -523,7 +523,7 @@ __device__ __forceinline__ bool bisect_node(BisectNode& N, const int* h, double 
       const int* c = hd[d] + (t - N.lo[d]);
       const int c0 = at_(c - 2), c1 = at_(c - 1), c2 = at_(c), c3 = at_(c + 1);
       const int a = c2 - 2 * c1 + c0, b = c3 - 2 * c2 + c1;
-      if (a * b < 0) {
+      if ((a < 0 && b > 0) || (a > 0 && b < 0)) {  // (a product of two counts can pass 32 bits)
         const unsigned long long v = ((unsigned long long)abs(a - b) << 42) | ((unsigned long long)(0x1fffff - abs(t - mid[d])) << 21) |
                                      (unsigned long long)(0x1fffff - t);
         key = v > key ? v : key;

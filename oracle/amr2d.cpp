@@ -2079,7 +2079,7 @@ struct Amr2 {
     for (int i = ilo + minoff; i <= ihi - minoff + 1; ++i) {
       const int t1 = iscr[i - 1], t2 = iscr[i];
       const int locdif = std::abs(t1 - t2);
-      if (t1 * t2 < 0) {
+      if ((t1 < 0 && t2 > 0) || (t1 > 0 && t2 < 0)) {  // (a product of two counts can pass 32 bits)
         if (locdif > locmaxi) { locmaxi = locdif; indexi = i; }
         else if (locdif == locmaxi) { if (std::abs(i - imid) < std::abs(indexi - imid)) indexi = i; }
       }
@@ -2091,7 +2091,7 @@ struct Amr2 {
     for (int j = jlo + minoff; j <= jhi - minoff + 1; ++j) {
       const int t1 = jscr[j - 1], t2 = jscr[j];
       const int locdif = std::abs(t1 - t2);
-      if (t1 * t2 < 0) {
+      if ((t1 < 0 && t2 > 0) || (t1 > 0 && t2 < 0)) {  // (a product of two counts can pass 32 bits)
         if (locdif > locmaxj) { locmaxj = locdif; indexj = j; }
         else if (locdif == locmaxj) { if (std::abs(j - jmid) < std::abs(indexj - jmid)) indexj = j; }
       }

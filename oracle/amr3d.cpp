@@ -2387,7 +2387,7 @@ struct Amr3 {
       locmax = 0; idx = 0; mid = (lo + hi) / 2;
       for (int i = lo + minoff; i <= hi - minoff + 1; ++i) {
         const int t1 = s[i - 1], t2 = s[i], d = std::abs(t1 - t2);
-        if (t1 * t2 < 0) {
+        if ((t1 < 0 && t2 > 0) || (t1 > 0 && t2 < 0)) {  // (a product of two counts can pass 32 bits)
           if (d > locmax) { locmax = d; idx = i; }
           else if (d == locmax && std::abs(i - mid) < std::abs(idx - mid)) idx = i;
         }
