@@ -128,14 +128,17 @@ struct Euler3Phys {
     euler3d_rpn_roe((T)sp.gamma, (T)sp.gamma1, sp.efix != 0, DIR, QL, QR, R, W, S, AM, AP);
     rc = split_recip(R.a);
   }
-  // FAST: the splits of euler3d_split_sub, for interfaces that quick() accepts
-  static constexpr bool HAS_QUICK = true;
+  template <int DIR>
+  __device__ __forceinline__ void rpt(int, int icoor, const T* in, T* m, T* p) const { euler3d_trans<false>(R, rc, DIR, icoor, in, m, p); }
+  template <int DIR>
+  __device__ __forceinline__ void rptt(int, int icoor, int, const T* in, T* m, T* p) const { euler3d_trans<false>(R, rc, DIR, icoor, in, m, p); }
+  // the quick form: euler3d_split_sub
   template <int DIR>
   __device__ __forceinline__ bool quick() const { return euler3d_trans_sub(R, DIR); }
-  template <int DIR, bool FAST = false>
-  __device__ __forceinline__ void rpt(int, int icoor, const T* in, T* m, T* p) const { euler3d_trans<FAST>(R, rc, DIR, icoor, in, m, p); }
-  template <int DIR, bool FAST = false>
-  __device__ __forceinline__ void rptt(int, int icoor, int, const T* in, T* m, T* p) const { euler3d_trans<FAST>(R, rc, DIR, icoor, in, m, p); }
+  template <int DIR>
+  __device__ __forceinline__ void rpt_quick(int, int icoor, const T* in, T* m, T* p) const { euler3d_trans<true>(R, rc, DIR, icoor, in, m, p); }
+  template <int DIR>
+  __device__ __forceinline__ void rptt_quick(int, int icoor, int, const T* in, T* m, T* p) const { euler3d_trans<true>(R, rc, DIR, icoor, in, m, p); }
 };
 
 // Advection in a face-centred velocity field (aux 1..3 = u, v, w at the left x-, y- and
@@ -147,9 +150,6 @@ struct Euler3Phys {
 template <class T>
 struct Swirl3Phys {
   static constexpr int NV = 1, NW = 1;
-  static constexpr bool HAS_QUICK = false;
-  template <int DIR>
-  __device__ __forceinline__ bool quick() const { return false; }
   T un;
   // [0]: cell e-1, [1]: cell e. vy: y-like face velocity at (dy, dz) = (0,0), (+1,0),
   // (0,-1), (+1,-1), (0,+1), (+1,+1); vz: z-like one at (0,0), (0,+1), (-1,0), (-1,+1),
@@ -184,19 +184,36 @@ struct Swirl3Phys {
     AM[0] = dmin(un, T(0)) * W[0][0];
     AP[0] = dmax(un, T(0)) * W[0][0];
   }
-  template <int DIR, bool = false>
+  template <int DIR>
   __device__ __forceinline__ void rpt(int imp, int icoor, const T* in, T* m, T* p) const {
     const int c = imp - 1;
     if (icoor == 2) { m[0] = dmin(vy[c][0], T(0)) * in[0]; p[0] = dmax(vy[c][1], T(0)) * in[0]; }
     else { m[0] = dmin(vz[c][0], T(0)) * in[0]; p[0] = dmax(vz[c][1], T(0)) * in[0]; }
   }
-  template <int DIR, bool = false>
+  template <int DIR>
   __device__ __forceinline__ void rptt(int imp, int icoor, int impt, const T* in, T* m, T* p) const {
     const int c = imp - 1, o = impt == 1 ? 2 : 4;
     if (icoor == 2) { m[0] = dmin(vy[c][o], T(0)) * in[0]; p[0] = dmax(vy[c][o + 1], T(0)) * in[0]; }
     else { m[0] = dmin(vz[c][o], T(0)) * in[0]; p[0] = dmax(vz[c][o + 1], T(0)) * in[0]; }
   }
 };
+
+// Whether a plugin has the optional quick form of its splits (include/amrgpu_riemann.cuh);
+// without one the sweeps make the contract's calls alone.
+template <class PH, class = void>
+struct HasQuick : std::false_type {};
+template <class PH>
+struct HasQuick<PH, std::void_t<decltype(std::declval<const PH&>().template quick<1>())>> : std::true_type {};
+template <int DIR, bool FAST, class T, class PH>
+__device__ __forceinline__ void split_t(const PH& ph, int imp, int icoor, const T* in, T* m, T* p) {
+  if constexpr (FAST) ph.template rpt_quick<DIR>(imp, icoor, in, m, p);
+  else ph.template rpt<DIR>(imp, icoor, in, m, p);
+}
+template <int DIR, bool FAST, class T, class PH>
+__device__ __forceinline__ void split_tt(const PH& ph, int imp, int icoor, int impt, const T* in, T* m, T* p) {
+  if constexpr (FAST) ph.template rptt_quick<DIR>(imp, icoor, impt, in, m, p);
+  else ph.template rptt<DIR>(imp, icoor, impt, in, m, p);
+}
 
 // the registered 3D plugins satisfy the device plugin contract (include/amrgpu_riemann.cuh)
 static_assert(amrgpu_plugin::Check3D<Euler3Phys<double>, Step3Params, double>::value, "euler_roe_efix: rpn3/rpt3/rptt3 contract");
@@ -224,8 +241,8 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
   const T sdt = first ? dtdx : -dtdx;  // the second-order parts enter with opposite signs
   // z-like split of the fluctuation and of the second-order part
   T cm[NV], cp[NV], cmq[NV], cpq[NV];
-  ph.template rpt<DIR, FAST>(imp, 3, F, cm, cp);
-  if (m3 == 2) ph.template rpt<DIR, FAST>(imp, 3, CQ, cmq, cpq);
+  split_t<DIR, FAST>(ph, imp, 3, F, cm, cp);
+  if (m3 == 2) split_t<DIR, FAST>(ph, imp, 3, CQ, cmq, cpq);
   else {
 #pragma unroll
     for (int m = 0; m < NV; ++m) cmq[m] = cpq[m] = T(0);
@@ -243,12 +260,12 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
     if (m4 > 0) {
       T t[NV];
       dt_input<NV>(w3, cp, cpq, t);
-      ph.template rptt<DIR, FAST>(imp, 2, 2, t, P1, P2);
+      split_tt<DIR, FAST>(ph, imp, 2, 2, t, P1, P2);
       dt_input<NV>(w3, cm, cmq, t);
-      ph.template rptt<DIR, FAST>(imp, 2, 1, t, M1, M2);
+      split_tt<DIR, FAST>(ph, imp, 2, 1, t, M1, M2);
     }
     T bm[NV], bp[NV];
-    ph.template rpt<DIR, FAST>(imp, 2, F, bm, bp);
+    split_t<DIR, FAST>(ph, imp, 2, F, bm, bp);
 #pragma unroll
     for (int m = 0; m < NV; ++m) {
       T g01 = (first ? T(0) : G(1 * NV + m)) - T(0.5) * dtdx * bm[m];
@@ -277,7 +294,7 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
     }
     T bmq[NV], bpq[NV];
     if (m3 == 2) {
-      ph.template rpt<DIR, FAST>(imp, 2, CQ, bmq, bpq);
+      split_t<DIR, FAST>(ph, imp, 2, CQ, bmq, bpq);
 #pragma unroll
       for (int m = 0; m < NV; ++m) {
         G(4 * NV + m) = G(4 * NV + m) + sdt * bpq[m];
@@ -292,9 +309,9 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
     if (m4 > 0) {
       T t[NV];
       dt_input<NV>(w3, bp, bpq, t);
-      ph.template rptt<DIR, FAST>(imp, 3, 2, t, X1, X2);
+      split_tt<DIR, FAST>(ph, imp, 3, 2, t, X1, X2);
       dt_input<NV>(w3, bm, bmq, t);
-      ph.template rptt<DIR, FAST>(imp, 3, 1, t, Y1, Y2);
+      split_tt<DIR, FAST>(ph, imp, 3, 1, t, Y1, Y2);
     }
 #pragma unroll
     for (int m = 0; m < NV; ++m) {
@@ -332,7 +349,7 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
 // [NW*NV][SW_T], then (after they are read) the transverse terms [12*NV][SW_T] of the
 // tile's cells: the apdq side writes them, the amdq side of the next interface adds to
 // them there, and each cell's terms then go to the stash in one coalesced write
-template <int DIR, class T, class PH>
+template <int DIR, class T, class PH, bool QUICK = HasQuick<PH>::value>
 __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, T (*sW)[SW_T]) {
   constexpr int NV = PH::NV, NW = PH::NW;
   T* const sG = &sW[0][0];
@@ -386,7 +403,7 @@ __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, 
   }
   // (a plugin with a quick form of its splits takes it where every interface of the tile may)
   bool quick = false;
-  if constexpr (PH::HAS_QUICK) quick = __syncthreads_and(!valid || ph.template quick<DIR>());
+  if constexpr (QUICK) quick = __syncthreads_and(!valid || ph.template quick<DIR>());
   else __syncthreads();
   // interfaces 1..n1+1 carry fluxes; the tile edges only serve their neighbours
   const bool live = valid && e >= 1 && e <= n1 + 1 && l >= 1 && l <= SW_T - 2;
@@ -451,7 +468,7 @@ __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, 
     __syncthreads();
     if (live && m3 > 0 && e >= 2 && l >= 2) trans_side<DIR, F, T, PH>(ph, 1, AM, CQ, m3, m4, dtdx, dtdy, dtdz, sG + (l - 1));
   };
-  if constexpr (PH::HAS_QUICK) {
+  if constexpr (QUICK) {
     if (quick) transverse(std::true_type{});
     else transverse(std::false_type{});
   } else transverse(std::false_type{});

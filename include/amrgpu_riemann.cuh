@@ -40,6 +40,14 @@
  *                                           R* m, R* p) const;
  *       DIR = ixyz; icoor 2: the y-like, 3: the z-like transverse direction of the sweep;
  *       impt: the side (1 minus, 2 plus) of the first transverse split.
+ *   template <int DIR> __device__ void load_normal(pool, patch, base, step, plane, e);
+ *       only for dimensionally split runs: as load, but what rpn alone needs (the rows beside
+ *       the pencil may lie outside the patch there).
+ *   A 3D plugin may also have a quick form of its splits with the same results, which the
+ *   sweeps take for a tile whose interfaces all allow it:
+ *   template <int DIR> __device__ bool quick() const;
+ *   template <int DIR> __device__ void rpt_quick(...) const, rptt_quick(...) const, with the
+ *   arguments of rpt and rptt.
  *
  * Every expression of a plugin must be evaluated in a fixed order (the library is built
  * without FMA contraction) so FP64 results are bit-identical to the CPU restatement.
