@@ -352,14 +352,20 @@ namespace {
 // the box, each warp takes i-rows (fixed j, k) of it in turn, 32 cells of a row at a time
 // (lane = i, coalesced reads). The i-counts go to shared memory one lane per bin; the j-
 // and k-counts of a chunk are summed across the warp first and added once. Counts are
-// integers, so the order of the adds does not matter.
+// integers, so the order of the adds does not matter. SH: a box's counts fit in shared memory
+// (12288 of them); longer boxes are counted in place.
+template <bool SH>
 __global__ void signatures3_kernel(const int8_t* f, LvlDims d, const SigBox* boxes, const int* off, int* hist) {
-  extern __shared__ int sh[];
+  extern __shared__ int block_counts[];
   const SigBox B = boxes[blockIdx.y];
   const int ni = B.hi[0] - B.lo[0] + 1, nj = B.hi[1] - B.lo[1] + 1, nk = B.hi[2] - B.lo[2] + 1;
   const int nh = ni + nj + nk;
-  for (int t = threadIdx.x; t < nh; t += blockDim.x) sh[t] = 0;
-  __syncthreads();
+  int* const h = hist + off[blockIdx.y];
+  int* const sh = SH ? block_counts : h;
+  if (SH) {
+    for (int t = threadIdx.x; t < nh; t += blockDim.x) sh[t] = 0;
+    __syncthreads();
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const long long rows = (long long)nj * nk;
   for (long long r = (long long)blockIdx.x * nwarps + warp; r < rows; r += (long long)gridDim.x * nwarps) {
@@ -377,8 +383,8 @@ __global__ void signatures3_kernel(const int8_t* f, LvlDims d, const SigBox* box
       atomicAdd(&sh[ni + nj + k], cnt);
     }
   }
+  if (!SH) return;
   __syncthreads();
-  int* h = hist + off[blockIdx.y];
   for (int t = threadIdx.x; t < nh; t += blockDim.x)
     if (sh[t]) atomicAdd(&h[t], sh[t]);
 }
@@ -402,7 +408,8 @@ void launch_signatures3(const int8_t* f, LvlDims d, const SigBox* boxes, int nbo
   const int slabs = (int)std::max<long long>(1, std::min<long long>(64, (maxrows + 7) / 8));
   for (int base = 0; base < nbox; base += 65535) {
     const int cnt = std::min(65535, nbox - base);
-    signatures3_kernel<<<dim3(slabs, cnt), 256, sizeof(int) * (size_t)maxlen, s>>>(f, d, boxes + base, off + base, hist);
+    if (maxlen <= 12288) signatures3_kernel<true><<<dim3(slabs, cnt), 256, sizeof(int) * (size_t)maxlen, s>>>(f, d, boxes + base, off + base, hist);
+    else signatures3_kernel<false><<<dim3(slabs, cnt), 256, 0, s>>>(f, d, boxes + base, off + base, hist);
   }
   AMR_CUDA(cudaGetLastError());
 }
