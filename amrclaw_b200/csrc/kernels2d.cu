@@ -15,7 +15,6 @@
 //   upbnd/average  level sync (upbnd.f:18-127, update.f:95-175).
 #include "kernels2d.cuh"
 #include <algorithm>
-#include <type_traits>
 
 namespace amrb {
 
@@ -78,6 +77,17 @@ __host__ __device__ constexpr int stage_row() {
 // the 600 substeps of a 100^2 quadrants run; one round of 352 threads takes 27 us, and 20 us
 // became 13 us for the mapped-grid advection. A uniform 1002^2 Euler level (3969 tiles) went
 // from 0.87 to 0.45 ms (one B200).
+// Waves of a face that the shared array holds at once: all of them, unless a double tile of
+// `rest` elements and `per_wave` more for each wave then takes more shared memory than a block
+// may have; the limiter goes through the waves in groups then (`least`: what the array has
+// for other uses anyway). All waves of every plugin here fit; a split step of 8 equations and
+// 5 waves, say, takes 246 KB with all of them and 222 KB with four.
+constexpr int wave_group(int waves, int per_wave, int least, int rest) {
+  int g = waves;
+  while (g > 1 && rest + (g * per_wave > least ? g * per_wave : least) > (232448 - 1024) / 8) --g;
+  return g;
+}
+
 template <class S>
 struct Step2Layout {
   static constexpr int ME = S::MEQN, MW = S::MWAVES;
@@ -87,10 +97,11 @@ struct Step2Layout {
   static constexpr int PITCH = (NLINE * NFACE + 3) / 4 * 4;  // elements of one shared value over the faces
   static constexpr int NQ = ME * QW * QW;
   static constexpr int NF = ME * (T + 1) * T;
-  static constexpr int NX = (MW * ME > 4 * ME ? MW * ME : 4 * ME) * PITCH;  // waves, then split results
   // aux of the tile and its two ghost layers, [m][b][a] like the staged q (solvers that read aux)
   static constexpr int NA = S::NAUX > 0 ? MAXAUX2 : 0;
   static constexpr int NAQ = NA * QW * QW;
+  static constexpr int WG = wave_group(MW, ME * PITCH, 4 * ME * PITCH, NQ + 4 * NF + NAQ + 32);
+  static constexpr int NX = (WG > 4 ? WG : 4) * ME * PITCH;  // waves, then split results
   static constexpr int TOTAL = NQ + 4 * NF + NX + NAQ + 32;
   static_assert(NLINE * NFACE <= STEP2_THREADS, "a thread per face of a sweep");
 };
@@ -118,28 +129,25 @@ __device__ __forceinline__ R philim2(int meth, R r) {
   return R(0);
 }
 
-// flux2.f:136-194 at one face whose waves, and those of the faces before and after it along
-// the line (threads tid -+ nb), are in X: limited waves, the second-order correction cq,
-// fm = (0 + amdq) + cq/2 and fp = (0 - apdq) + cq/2. dl, dr: dtdx1d of the cells left and
-// right of the face (dt/dx, divided by the capacity of the cell when there is one:
-// step2.f90:83-88)
-template <class S, class R>
-__device__ __forceinline__ void limited_fluxes(const StepParams& sp, const R* X, int pitch, int tid, int nb, R dl, R dr,
-                                               const R (&s)[S::MWAVES], const R (&amdq)[S::MEQN], const R (&apdq)[S::MEQN],
-                                               R (&cq)[S::MEQN], R (&fm)[S::MEQN], R (&fp)[S::MEQN]) {
+// limiter.f and the second-order correction of flux2.f:136-194 for the waves w0 .. w0+G-1 of
+// one face, added to cq. They, and those of the faces before and after it along the line
+// (threads tid -+ nb), are in X. dl, dr: dtdx1d of the cells left and right of the face (dt/dx,
+// divided by the capacity of the cell when there is one: step2.f90:83-88)
+template <class S, int G, class R>
+__device__ __forceinline__ void limited_waves(const StepParams& sp, const R* X, int pitch, int tid, int nb, R dl, R dr, int w0,
+                                              const R (&s)[S::MWAVES], R (&cq)[S::MEQN]) {
   constexpr int ME = S::MEQN, MW = S::MWAVES;
-#pragma unroll
-  for (int m = 0; m < ME; ++m) { cq[m] = R(0); fm[m] = R(0) + amdq[m]; fp[m] = R(0) - apdq[m]; }
-  if (sp.order == 1) return;
   const R dtdxave = R(0.5) * (dl + dr);
 #pragma unroll
-  for (int mw = 0; mw < MW; ++mw) {
+  for (int g = 0; g < G; ++g) {
+    const int mw = w0 + g;
+    if (mw >= MW) break;
     R w[ME];
 #pragma unroll
-    for (int m = 0; m < ME; ++m) w[m] = X[(mw * ME + m) * pitch + tid];
+    for (int m = 0; m < ME; ++m) w[m] = X[(g * ME + m) * pitch + tid];
     if (sp.mthlim[mw] != 0) {
       // the ratio takes the neighbour on the upwind side
-      const R* wn = X + mw * ME * pitch + tid + (s[mw] > R(0) ? -nb : nb);
+      const R* wn = X + g * ME * pitch + tid + (s[mw] > R(0) ? -nb : nb);
       R wn2 = R(0), dot = R(0);
 #pragma unroll
       for (int m = 0; m < ME; ++m) { wn2 = wn2 + w[m] * w[m]; dot = dot + wn[m * pitch] * w[m]; }
@@ -153,8 +161,72 @@ __device__ __forceinline__ void limited_fluxes(const StepParams& sp, const R* X,
 #pragma unroll
     for (int m = 0; m < ME; ++m) cq[m] = cq[m] + c * w[m];
   }
+}
+
+// waves w0 .. w0+G-1 of a thread's face into X
+template <int G, class R, int MW, int ME>
+__device__ __forceinline__ void share_waves(R* X, int pitch, int tid, int w0, const R (&wave)[MW][ME]) {
 #pragma unroll
-  for (int m = 0; m < ME; ++m) { fm[m] = fm[m] + R(0.5) * cq[m]; fp[m] = fp[m] + R(0.5) * cq[m]; }
+  for (int g = 0; g < G; ++g)
+#pragma unroll
+    for (int m = 0; m < ME; ++m)
+      if (w0 + g < MW) X[(g * ME + m) * pitch + tid] = wave[w0 + g][m];
+}
+
+// What a face keeps of its waves between its Riemann problem and limited_fluxes: nothing where
+// X holds all of them, else the waves themselves.
+template <class S, int WG, class R>
+struct WaveKeep {
+  static constexpr int MW = S::MWAVES, ME = S::MEQN;
+  static constexpr bool WHOLE = WG >= MW;
+  R wave[WHOLE ? 1 : MW][ME], cq[ME];
+  // an active thread, with the waves of its face
+  __device__ __forceinline__ void put(R* X, int pitch, int tid, const R (&w)[MW][ME]) {
+    if constexpr (WHOLE) share_waves<MW>(X, pitch, tid, 0, w);
+    else {
+#pragma unroll
+      for (int k = 0; k < MW; ++k)
+#pragma unroll
+        for (int m = 0; m < ME; ++m) wave[k][m] = w[k][m];
+    }
+  }
+  // every thread of the block, then: after it the waves of all faces, or the corrections of
+  // this one, are there
+  __device__ __forceinline__ void meet(const StepParams& sp, R* X, int pitch, int tid, int nb, bool active, bool flux, R dl, R dr,
+                                       const R (&s)[MW]) {
+    if constexpr (!WHOLE) {
+#pragma unroll
+      for (int m = 0; m < ME; ++m) cq[m] = R(0);
+#pragma unroll
+      for (int w0 = 0; w0 < MW; w0 += WG) {
+        if (w0 > 0) __syncthreads();  // the group before is read
+        if (active) share_waves<WG>(X, pitch, tid, w0, wave);
+        __syncthreads();
+        if (flux && sp.order != 1) limited_waves<S, WG, R>(sp, X, pitch, tid, nb, dl, dr, w0, s, cq);
+      }
+    } else {
+      __syncthreads();
+    }
+  }
+};
+
+// flux2.f:136-194 at one face: the second-order correction c, fm = (0 + amdq) + c/2 and
+// fp = (0 - apdq) + c/2
+template <class S, int WG, class R>
+__device__ __forceinline__ void limited_fluxes(const WaveKeep<S, WG, R>& keep, const StepParams& sp, const R* X, int pitch, int tid,
+                                               int nb, R dl, R dr, const R (&s)[S::MWAVES], const R (&amdq)[S::MEQN],
+                                               const R (&apdq)[S::MEQN], R (&c)[S::MEQN], R (&fm)[S::MEQN], R (&fp)[S::MEQN]) {
+  constexpr int ME = S::MEQN;
+#pragma unroll
+  for (int m = 0; m < ME; ++m) { c[m] = R(0); fm[m] = R(0) + amdq[m]; fp[m] = R(0) - apdq[m]; }
+  if (sp.order == 1) return;
+  if constexpr (WaveKeep<S, WG, R>::WHOLE) limited_waves<S, S::MWAVES, R>(sp, X, pitch, tid, nb, dl, dr, 0, s, c);
+  else {
+#pragma unroll
+    for (int m = 0; m < ME; ++m) c[m] = keep.cq[m];
+  }
+#pragma unroll
+  for (int m = 0; m < ME; ++m) { fm[m] = fm[m] + R(0.5) * c[m]; fp[m] = fp[m] + R(0.5) * c[m]; }
 }
 
 // One sweep direction of flux2.f over the tile. IXY = 1: lines are rows, IXY = 2: columns.
@@ -192,6 +264,7 @@ __device__ __forceinline__ void step2_sweep(const StepParams& sp, const R* Qs, c
   // dtdx1d of a cell (step2.f90:83-88)
   auto d1d = [&](int ln, int pos) -> R { return capa ? dtdx / As[at(sp.mcapa - 1, ln, pos)] : dtdx; };
   Iface2<S, R> face;
+  WaveKeep<S, L::WG, R> keep;
   R s[MW], amdq[ME], apdq[ME];
   R dl = dtdx, dr = dtdx;
   // the normal Riemann problem: waves to the shared array
@@ -203,23 +276,20 @@ __device__ __forceinline__ void step2_sweep(const StepParams& sp, const R* Qs, c
     auxc(aR, line + 1, ff + 1);
     face.rpn(sp.prob, IXY, qL, qR, aL.v, aR.v, wave, s, amdq, apdq);
     dl = d1d(line + 1, ff); dr = d1d(line + 1, ff + 1);
-#pragma unroll
-    for (int mw = 0; mw < MW; ++mw)
-#pragma unroll
-      for (int m = 0; m < ME; ++m) X[(mw * ME + m) * PITCH + tid] = wave[mw][m];
+    keep.put(X, PITCH, tid, wave);
     if (ff >= 1 && ff <= na + 1) {
 #pragma unroll
       for (int mw = 0; mw < MW; ++mw) cfl = dmax(cfl, dmax(dr * s[mw], -dl * s[mw]));
     }
   }
-  __syncthreads();
-  // limiter, second-order correction (flux2.f:136-194), face fluxes of the tile's own lines
   const bool flux = active && ff >= 1 && ff <= na + 1;
   const bool split = flux && sp.trans != 0;
+  keep.meet(sp, X, PITCH, tid, IXY == 1 ? 1 : L::NLINE, active, flux, dl, dr, s);
+  // limiter, second-order correction (flux2.f:136-194), face fluxes of the tile's own lines
   R am2[ME], ap2[ME];
   if (flux) {
     R cq[ME], fm[ME], fp[ME];
-    limited_fluxes<S, R>(sp, X, PITCH, tid, IXY == 1 ? 1 : L::NLINE, dl, dr, s, amdq, apdq, cq, fm, fp);
+    limited_fluxes<S, L::WG, R>(keep, sp, X, PITCH, tid, IXY == 1 ? 1 : L::NLINE, dl, dr, s, amdq, apdq, cq, fm, fp);
     const int lin = line - 1, fa = ff - 1;
     if (lin >= 0 && lin < nt) {
 #pragma unroll
@@ -464,12 +534,13 @@ __device__ __forceinline__ bool step2_tile(const StepArgs& a, const StepWork& wk
 }
 
 // Resident tiles per SM that the register budget is sized for. Two tiles leave a thread 80
-// registers: enough for every solver but Euler in FP64, which then spills and takes 41 us
+// registers. A thread holds the waves of its face: up to 64 bytes of them (FP32 Euler, which
+// spills 108 bytes) two tiles fit; FP64 Euler, with 128, spills 860 bytes and takes 41 us
 // instead of 30 us for a level of some 60-120 tiles (24.3 against 18.1 ms over the 600
 // substeps of a 100^2 quadrants run), and gains nothing on a level of 3969 tiles.
 template <class S, class R>
 constexpr int step2_blocks() {
-  return std::is_same<S, Euler2>::value && sizeof(R) == 8 ? 1 : 2;
+  return S::MWAVES * S::MEQN * (int)sizeof(R) <= 64 ? 2 : 1;
 }
 
 // the bulk-copy barrier of a step block: one arrival per phase (thread 0), the rows' bytes
@@ -558,9 +629,10 @@ struct Split2Layout {
   static constexpr int NFX = ME * QW * (T + 1);      // fm / fp of every staged row
   static constexpr int NQX = ME * QW * T;            // x-updated q of the tile's columns
   static constexpr int NG = ME * (T + 1) * T;        // gm / gp
-  static constexpr int NX = MW * ME * PITCH;         // waves
   static constexpr int NA = S::NAUX > 0 ? MAXAUX2 : 0;
   static constexpr int NAQ = NA * QW * QW;           // staged aux, [m][b][a] like Qs
+  static constexpr int WG = wave_group(MW, ME * PITCH, 0, NQ + 2 * NFX + NQX + 2 * NG + NAQ + 32);
+  static constexpr int NX = WG * ME * PITCH;         // waves
   static constexpr int TOTAL = NQ + 2 * NFX + NQX + 2 * NG + NX + NAQ + 32;
   static_assert(PITCH <= SPLIT2_THREADS, "a thread per face of a sweep");
 };
@@ -574,30 +646,28 @@ __device__ __forceinline__ void split2_round(const StepParams& sp, R* X, int pit
                                              R (&fm)[S::MEQN], R (&fp)[S::MEQN]) {
   constexpr int ME = S::MEQN, MW = S::MWAVES;
   const int tid = threadIdx.x;
+  WaveKeep<S, Split2Layout<S>::WG, R> keep;
   R s[MW], amdq[ME], apdq[ME];
   if (active) {
     R qL[ME], qR[ME], wave[MW][ME];
 #pragma unroll
     for (int m = 0; m < ME; ++m) { qL[m] = ql(m); qR[m] = qr(m); }
     S::template rpn<R>(sp.prob, IXY, qL, qR, aL.v, aR.v, wave, s, amdq, apdq);
-#pragma unroll
-    for (int mw = 0; mw < MW; ++mw)
-#pragma unroll
-      for (int m = 0; m < ME; ++m) X[(mw * ME + m) * pitch + tid] = wave[mw][m];
+    keep.put(X, pitch, tid, wave);
     if (flux) {
 #pragma unroll
       for (int mw = 0; mw < MW; ++mw) cfl = dmax(cfl, dmax(dr * s[mw], -dl * s[mw]));
     }
   }
-  __syncthreads();
+  keep.meet(sp, X, pitch, tid, nb, active, flux, dl, dr, s);
   if (flux) {
     R cq[ME];
-    limited_fluxes<S, R>(sp, X, pitch, tid, nb, dl, dr, s, amdq, apdq, cq, fm, fp);
+    limited_fluxes<S, Split2Layout<S>::WG, R>(keep, sp, X, pitch, tid, nb, dl, dr, s, amdq, apdq, cq, fm, fp);
   }
 }
 
 template <class S, class R>
-__global__ void __launch_bounds__(SPLIT2_THREADS, std::is_same<S, Euler2>::value && sizeof(R) == 8 ? 1 : 2) step2s_kernel(StepArgs a) {
+__global__ void __launch_bounds__(SPLIT2_THREADS, (step2_blocks<S, R>())) step2s_kernel(StepArgs a) {
   using L = Split2Layout<S>;
   constexpr int ME = L::ME, T = L::T, QW = L::QW, NFACE = L::NFACE;
   extern __shared__ __align__(16) unsigned char smem_raw[];

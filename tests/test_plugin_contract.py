@@ -33,6 +33,39 @@ template int launch_step3_t<float, Contract3<float>>(const Step3Args&, const lon
 }
 """
 
+PLUGIN2 = """
+#include "kernels2d.cu"
+namespace amrb {
+template <int NE, int NWV>
+struct Contract2 {
+  static constexpr int MEQN = NE, MWAVES = NWV, NAUX = 0;
+  template <class R>
+  __device__ static void rpn(const ProbDev&, int, const R* qL, const R* qR, const R*, const R*, R (&wave)[MWAVES][MEQN],
+                             R (&s)[MWAVES], R (&amdq)[MEQN], R (&apdq)[MEQN]) {
+    for (int k = 0; k < MWAVES; ++k) { s[k] = R(1); for (int m = 0; m < MEQN; ++m) wave[k][m] = (qR[m] - qL[m]) / R(MWAVES); }
+    for (int m = 0; m < MEQN; ++m) { amdq[m] = R(0); apdq[m] = qR[m] - qL[m]; }
+  }
+  template <class R>
+  __device__ static void rpt(const ProbDev&, int, int, const R*, const R*, const R*, const R*, const R*, const R* asdq,
+                             R (&bm)[MEQN], R (&bp)[MEQN]) {
+    for (int m = 0; m < MEQN; ++m) { bm[m] = R(0); bp[m] = asdq[m]; }
+  }
+};
+// a block's shared memory holds a tile of these, as it did with the tile's waves in chunks of rows
+template <class S> constexpr bool unsplit_fits() { return Step2Layout<S>::TOTAL * 8 <= 232448 - 512; }
+template <class S> constexpr bool split_fits() { return Split2Layout<S>::TOTAL * 8 <= 232448 - 512; }
+static_assert(unsplit_fits<Contract2<8, 7>>() && unsplit_fits<Contract2<8, 5>>() && unsplit_fits<Contract2<10, 1>>(), "");
+static_assert(split_fits<Contract2<7, 7>>() && split_fits<Contract2<8, 7>>() && split_fits<Contract2<10, 5>>(), "");
+static_assert(split_fits<Contract2<11, 3>>() && split_fits<Contract2<12, 1>>(), "");
+// the plugins of this library have all their waves there at once
+static_assert(Step2Layout<Euler2>::WG == 4 && Split2Layout<Euler2>::WG == 4 && Split2Layout<Acoustics2>::WG == 2, "");
+static_assert(amrgpu_plugin::Check2D<Contract2<8, 5>, ProbDev, double>::value, "");
+template void launch_step2_t<Contract2<8, 5>, double>(const StepArgs&, int, cudaStream_t);
+template void launch_step2_t<Contract2<8, 5>, float>(const StepArgs&, int, cudaStream_t);
+template void launch_step2_batch_t<Contract2<8, 5>, double>(const StepBatch&, int, cudaStream_t);
+}
+"""
+
 
 def _front_end(src):
     """Compiles to intermediate code without optimising it (nothing is kept)."""
@@ -46,4 +79,9 @@ def _front_end(src):
 
 def test_3d_plugin_of_the_contract_alone():
     rc, err = _front_end(PLUGIN3.replace("const long long*", "const long long*"))
+    assert rc == 0, err
+
+
+def test_2d_plugin_of_the_contract_alone():
+    rc, err = _front_end(PLUGIN2)
     assert rc == 0, err
