@@ -381,7 +381,7 @@ __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, 
     const unsigned loc = (unsigned)(g - c0[pi]), pen = loc / (unsigned)(n1 + 3);
     e = (int)(loc - pen * (unsigned)(n1 + 3));
     const int b = (int)(pen / (unsigned)(n2 + 2)), a = (int)(pen - (unsigned)b * (unsigned)(n2 + 2));
-    slot = s0[pi] + pen * pencil_slots(n1) + (e - 1);
+    slot = s0[pi] + pen * pencil_slots(n1, A.pad) + (e - 1);
     const long long mi = P.mitot, mj = P.mjtot;
     long long base, step;  // enlarged-array index of pencil cell x is base + x*step (cell 0: enlarged index 1)
     if (DIR == 1) { base = ((long long)(b - 1 + NG3) * mj + (a - 1 + NG3)) * mi + (NG3 - 1); step = 1; }
@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(128) face3_kernel(Step3Args A) {
     const int i0 = r3 % icnt, j0 = (r3 / icnt) % jcnt, k0 = r3 / (icnt * jcnt);
     const int i = ib * FB_I + i0 + 1, j = jb * FB_J + j0 + 1, k = kb * FB_K + k0 + 1;
     const long long bx = A.sweep0[pi], by = A.sweep0[(A.np + 1) + pi], bz = A.sweep0[2 * (A.np + 1) + pi];
-    const int px = (int)pencil_slots(mx), py = (int)pencil_slots(my), pz = (int)pencil_slots(mz);
+    const int px = (int)pencil_slots(mx, A.pad), py = (int)pencil_slots(my, A.pad), pz = (int)pencil_slots(mz, A.pad);
     auto xs = [&](int jj, int kk, int ii) { return stash_at<NV>(bx + ((long long)(kk * (my + 2) + jj) * px + (ii - 1))); };
     auto ys = [&](int ii, int kk, int jj) { return stash_at<NV>(by + ((long long)(kk * (mx + 2) + ii) * py + (jj - 1))); };
     auto zs = [&](int ii, int jj, int kk) { return stash_at<NV>(bz + ((long long)(jj * (mx + 2) + ii) * pz + (kk - 1))); };

@@ -11,11 +11,12 @@ __host__ __device__ constexpr int stash_values(int nv) { return 14 * nv; }
 constexpr int STASH3 = stash_values(5);
 // Layout of the stash: blocks of 32 slots, [slot / 32][stash_values][slot % 32], so that the
 // values of a slot lie at constant distances. A pencil of n1 cells (n1+1 interfaces) takes
-// whole groups of 8 slots: the face kernel takes its faces in blocks of four or eight along
-// an axis, and eight consecutive interfaces of a pencil, counted from its first, then are
-// one whole 64-byte piece of DRAM (double), read once.
+// whole groups of 8 slots (pad 7): the face kernel takes its faces in blocks of four or eight
+// along an axis, and eight consecutive interfaces of a pencil, counted from its first, then are
+// one whole 64-byte piece of DRAM (double), read once. Where the stash has no room for that the
+// pencils of a level lie one after the other (pad 0).
 constexpr int STASH_BLK = 32;
-__host__ __device__ constexpr long long pencil_slots(long long n1) { return (n1 + 8) & ~7LL; }
+__host__ __device__ constexpr long long pencil_slots(long long n1, int pad) { return (n1 + 1 + pad) & ~(long long)pad; }
 // slots of a level (the sum of its pencils') in whole blocks
 __host__ __device__ constexpr long long stash_slots(long long n) { return (n + STASH_BLK - 1) & ~(long long)(STASH_BLK - 1); }
 template <int NV>
@@ -43,11 +44,12 @@ struct Step3Args {
   const PatchDev* patches;
   const int* plist;          // patch ids of the level, in level order
   int np;
-  const long long* sweep0;   // [3][np+1]: first stash slot of each patch, per direction (pencil_slots(n1) per pencil)
+  const long long* sweep0;   // [3][np+1]: first stash slot of each patch, per direction (pencil_slots(n1, pad) per pencil)
   const long long* comp0;    // [3][np+1]: first interface of each patch, per direction ((n1+3) per pencil)
   const long long* face0;    // [np+1]: first face cell of each patch ((mx+1)(my+1)(mz+1) each)
   const long long* cell0;    // [np+1]: first interior cell of each patch (mx*my*mz each)
   void* stash;               // see stash_at
+  int pad;                   // of the pencils in the stash: 7 or 0
   void* flux;                // [6 comps][meqn][face cells]
   long long flux_stride;     // face cells of the level
   double dt, dx, dy, dz;
