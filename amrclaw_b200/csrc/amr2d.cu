@@ -2067,13 +2067,14 @@ class Amr2Gpu {
 
   // ---------------------------------------------------------------- clustering
   // Berger-Rigoutsos bisection (smartbis.f:25-177, signs.f:16-71, findcut.f:7-130,
-  // moment.f:16-75) driven by signatures made on the device. The level's points (the
-  // buffered, nested, wrapped and deduplicated flags of flag_points) are scattered into a
-  // one-plane device array; a cluster is a box of it and its points the flagged cells
-  // inside. Each wave of the bisection sends the boxes of all undecided clusters to the
-  // device, which counts the points per i and per j of every box; only those counts come
-  // back, and the host takes from them the count, the bounding box, the efficiency and the
-  // cut. Every decision depends only on these counts, as the reference's do on its points.
+  // moment.f:16-75) of the level's points: the buffered, nested, wrapped and deduplicated
+  // flags of flag_points. One launch takes the list of points and makes the whole tree
+  // (DeviceBisect). Past its limits, and for the splits of nestck2, the points are scattered
+  // into a one-plane device array; a cluster is a box of it and its points the flagged cells
+  // inside. The device counts the points per i and per j of every box sent (a wave of the
+  // bisection at a time), only those counts come back, and the host takes from them the
+  // count, the bounding box, the efficiency and the cut. In both forms every decision depends
+  // only on these counts, as the reference's do on its points.
   struct Clu2 { SigBox box; int n = 0; int lo[2] = {0, 0}, hi[2] = {0, 0}; };
   DBuf<int8_t> sig_mask;
   DBuf<int> sig_pts, sig_off, sig_hist;
@@ -2141,18 +2142,22 @@ class Amr2Gpu {
   // moment.f: rect (0-based level indices ilo, ihi, jlo, jhi) and efficiency of a cluster
   static double moment2(const Clu2& c, int rect[4]) {
     rect[0] = c.lo[0] - 1; rect[1] = c.hi[0] - 1; rect[2] = c.lo[1] - 1; rect[3] = c.hi[1] - 1;
-    return (double)c.n / (double)((rect[1] - rect[0] + 1) * (rect[3] - rect[2] + 1));
+    return (double)c.n / (double)((long long)(rect[1] - rect[0] + 1) * (rect[3] - rect[2] + 1));
   }
-  // smartbis.f in one launch (DeviceBisect); past its limits breadth first over the device
+  // smartbis.f in one launch (DeviceBisect); past its limits breadth first over the device's
   // signatures. Leaves in the reference's order (the part at or above the cut first)
   std::vector<Clu2> bisect_on_device(const std::vector<Pt>& pts, int lcheck, double cutoff) {
     sig_dims = LvlDims{iregsz[lcheck], jregsz[lcheck], 1};
     sig_points = &pts;
-    std::vector<unsigned long long> list(pts.size());
-    for (size_t k = 0; k < pts.size(); ++k) list[k] = bisect_point(pts[k].i + 1, pts[k].j + 1, 1);
+    std::vector<unsigned long long> list;
+    if (DeviceBisect::takes(2, sig_dims, pts.size())) {
+      list.resize(pts.size());
+      for (size_t k = 0; k < pts.size(); ++k) list[k] = bisect_point(pts[k].i + 1, pts[k].j + 1, 1);
+    }
     std::vector<BisectNode> tree;
-    nkernels += 2;
-    if (bis.run(2, nullptr, sig_dims, list, cutoff, st, stg, tree)) {
+    const bool done = !list.empty() && bis.run(2, nullptr, sig_dims, list, cutoff, st, stg, tree);
+    if (!list.empty()) nkernels += bis.launched;
+    if (done) {
       std::vector<Clu2> out;
       for (int id : DeviceBisect::leaves(tree)) {
         const BisectNode& N = tree[id];

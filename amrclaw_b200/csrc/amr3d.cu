@@ -2056,8 +2056,8 @@ class Amr3Gpu : public AmrSolver {
   // moment.f:4-70: bounding box (rect: ilo, ihi, jlo, jhi, klo, khi, 0-based) and efficiency
   static void moment(int rect[6], const Clu3& c, double& usage) {
     for (int d = 0; d < 3; ++d) { rect[2 * d] = c.lo[d] - 1; rect[2 * d + 1] = c.hi[d] - 1; }
-    const int gpall = (rect[1] - rect[0] + 1) * (rect[3] - rect[2] + 1) * (rect[5] - rect[4] + 1);
-    usage = (double)c.n / gpall;
+    const long long gpall = (long long)(rect[1] - rect[0] + 1) * (rect[3] - rect[2] + 1) * (rect[5] - rect[4] + 1);
+    usage = (double)c.n / (double)gpall;
   }
   // findcut.f on a cluster's signatures scr (counts at level indices 0..dims+1): a hole in
   // a signature, else the largest Laplacian sign change (ties to the middle)
@@ -2099,14 +2099,15 @@ class Amr3Gpu : public AmrSolver {
   }
   // smartbis.f: bisect until every cluster's efficiency reaches cutoff or it has no cut, in
   // one launch (DeviceBisect); past its limits breadth first here, one signature wave per
-  // depth, then the leaves in the reference's
-  // depth-first order: the part at or above the cut before the part below it
+  // depth. Then the leaves in the reference's depth-first order: the part at or above the cut
+  // before the part below it
   DeviceBisect bis;
   std::vector<Clu3> cluster_on_device(double cutoff) {
     const int dims[3] = {lv_dims.is, lv_dims.js, lv_dims.ks};
     std::vector<BisectNode> tree;
-    nkernels += 3;
-    if (bis.run(3, lv_b.d, lv_dims, {}, cutoff, st, stg, tree)) {
+    const bool done = bis.run(3, lv_b.d, lv_dims, {}, cutoff, st, stg, tree);
+    nkernels += bis.launched;
+    if (done) {
       std::vector<Clu3> out;
       for (int id : DeviceBisect::leaves(tree)) {
         const BisectNode& N = tree[id];

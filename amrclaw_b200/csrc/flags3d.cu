@@ -445,8 +445,8 @@ __global__ void __launch_bounds__(256) list_points_kernel(const int8_t* f, LvlDi
 }
 
 // All blocks of the launch (co-resident: it is a cooperative one). False when a block gave up
-// waiting after about a second; every block then leaves.
-__device__ __forceinline__ bool bisect_barrier(BisectHead* h, unsigned& turn) {
+// waiting (max_wait); every block then leaves.
+__device__ __forceinline__ bool bisect_barrier(BisectHead* h, unsigned& turn, long long max_wait) {
   if (gridDim.x == 1) { __syncthreads(); return true; }
   __shared__ int ok;
   __syncthreads();
@@ -457,7 +457,7 @@ __device__ __forceinline__ bool bisect_barrier(BisectHead* h, unsigned& turn) {
     const long long t0 = clock64();
     ok = 1;
     while (*(volatile unsigned*)&h->arrived < turn * gridDim.x) {
-      if (clock64() - t0 > 2000000000LL) { ok = 0; break; }
+      if (clock64() - t0 > max_wait) { ok = 0; break; }
     }
     if (!ok) atomicExch(&h->stop, 2);
     __threadfence();
@@ -503,7 +503,7 @@ __device__ __forceinline__ bool bisect_node(BisectNode& N, const int* h, double 
   }
   N.n = n;
   if (n == 0) return false;
-  int vol = 1;
+  long long vol = 1;
 #pragma unroll
   for (int d = 0; d < ND; ++d) vol *= N.chi[d] - N.clo[d] + 1;
   if ((double)n / (double)vol >= cutoff) return false;
@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(BIS_THREADS) bisect_kernel(BisectArgs A) {
     A.nodes[0] = R;
     H->nodes = 1;
   }
-  if (!bisect_barrier(H, turn)) return;
+  if (!bisect_barrier(H, turn, A.max_wait)) return;
   int w0 = 0, w1 = 1, cur = 0;
   while (true) {
     if (tid == 0) H->hlen[cur ^ 1] = 0;
@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(BIS_THREADS) bisect_kernel(BisectArgs A) {
         }
       }
     }
-    if (!bisect_barrier(H, turn)) return;
+    if (!bisect_barrier(H, turn, A.max_wait)) return;
     int* next = A.hist + (long long)(cur ^ 1) * A.max_hist;
     for (int b = w0 + (int)warp; b < w1; b += (int)nwarps) {
       BisectNode N;
@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(BIS_THREADS) bisect_kernel(BisectArgs A) {
       }
       if (lane == 0) A.nodes[b] = N;
     }
-    if (!bisect_barrier(H, turn)) return;
+    if (!bisect_barrier(H, turn, A.max_wait)) return;
     if (*(volatile int*)&H->stop) return;
     w0 = w1;
     w1 = *(volatile int*)&H->nodes;
@@ -713,7 +713,7 @@ __global__ void __launch_bounds__(BIS_THREADS) bisect_kernel(BisectArgs A) {
 }
 }  // namespace
 
-void launch_bisect(int ndim, const BisectArgs& a, const int8_t* f, LvlDims d, unsigned npts, cudaStream_t s) {
+int launch_bisect(int ndim, const BisectArgs& a, const int8_t* f, LvlDims d, unsigned npts, cudaStream_t s) {
   bisect_head_kernel<<<1, 1, 0, s>>>(a.head, ndim == 3 ? 0u : npts);
   if (ndim == 3) {
     const long long cells = (long long)((d.is + 31) / 32 * 32) * d.js * d.ks;
@@ -725,11 +725,12 @@ void launch_bisect(int ndim, const BisectArgs& a, const int8_t* f, LvlDims d, un
   if (blocks == 1) {
     bisect_kernel<2><<<1, BIS_THREADS, 0, s>>>(a);
     AMR_CUDA(cudaGetLastError());
-    return;
+    return 2;
   }
   void* args[1] = {const_cast<BisectArgs*>(&a)};
   AMR_CUDA(cudaLaunchCooperativeKernel(ndim == 3 ? (const void*)bisect_kernel<3> : (const void*)bisect_kernel<2>, dim3(blocks),
                                        dim3(BIS_THREADS), args, 0, s));
+  return ndim == 3 ? 3 : 2;
 }
 
 // ======================================================================= Richardson estimation

@@ -79,10 +79,12 @@ struct BisectArgs {
   int* hist; int max_hist;      // two buffers of max_hist ints
   int dims[3];
   double cutoff;
+  long long max_wait;           // clock cycles after which a block stops waiting for the others
 };
+constexpr long long BISECT_MAX_WAIT = 2000000000;  // about a second
 // ndim 3: the points are the flagged cells (f != 0) of the level array's interior, listed on
-// the device first; ndim 2: npts points are already in a.pts.
-void launch_bisect(int ndim, const BisectArgs& a, const int8_t* f, LvlDims d, unsigned npts, cudaStream_t s);
+// the device first; ndim 2: npts points are already in a.pts. Returns the kernels launched.
+int launch_bisect(int ndim, const BisectArgs& a, const int8_t* f, LvlDims d, unsigned npts, cudaStream_t s);
 
 // 2D: the level's flag array as a one-plane array (d.ks = 1): zeroed, then 1 at every point
 // (pts: n pairs of 0-based level indices i, j) at array position (i+1, j+1, 1)

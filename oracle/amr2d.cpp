@@ -2053,7 +2053,7 @@ struct Amr2 {
     rect[0] = (int)std::nearbyint(emn1 - 0.5); rect[2] = (int)std::nearbyint(emn2 - 0.5);
     rect[1] = (int)std::nearbyint(emx1 - 0.5); rect[3] = (int)std::nearbyint(emx2 - 0.5);
     const int s1 = rect[1] - rect[0] + 1, s2 = rect[3] - rect[2] + 1;
-    usage = rn / (double)(s1 * s2);
+    usage = rn / (double)((long long)s1 * s2);
   }
   void signs(const double* badpts, int ist, int iend, std::vector<int>& iscr, std::vector<int>& jscr, int idim, int jdim,
              int& ilo, int& ihi, int& jlo, int& jhi) {

@@ -2360,7 +2360,7 @@ struct Amr3 {
     rect[2] = (int)std::lround(emn2 - .5); rect[3] = (int)std::lround(emx2 - .5);
     rect[4] = (int)std::lround(emn3 - .5); rect[5] = (int)std::lround(emx3 - .5);
     const int s1 = rect[1] - rect[0] + 1, s2 = rect[3] - rect[2] + 1, s3 = rect[5] - rect[4] + 1;
-    const int gpall = s1 * s2 * s3;
+    const long long gpall = (long long)s1 * s2 * s3;
     usage = (double)npt / gpall;
   }
   // signs.f:4-86 + findcut.f:4-198 ; returns index (0: none) and iside
