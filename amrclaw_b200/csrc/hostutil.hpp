@@ -206,8 +206,9 @@ inline void set_arena_limits(Arena& pool, Arena& regs, long long bytes) {
 // a few MB between two synchronisations. (One ring of 256 MB pinned at start-up cost a 3D
 // solve about 130 ms of its own.) The chain grows by what it holds up to `soon`; then it
 // synchronizes the stream and starts over when it is full, and grows again, up to LIMIT, each
-// time that has happened WRAPS times. A chunk is kept until the context ends, so growing
-// neither frees nor waits.
+// time that has happened WRAPS times. Growing up to LIMIT neither frees nor waits. Where the
+// chunk of one large upload would take the chain past LIMIT, the stream is synchronized and
+// the chunk takes the place of earlier ones; only an upload larger than LIMIT holds more.
 struct Staging {
   struct Chunk { char* h; size_t cap; };
   static constexpr size_t FIRST = (size_t)1 << 20, LIMIT = (size_t)256 << 20;
@@ -230,11 +231,22 @@ struct Staging {
       seek(n2);
     }
     if (at == chunks.size()) {
-      const size_t cap = std::max<size_t>({n2, std::min(held, LIMIT - std::min(held, LIMIT)), FIRST});
+      const size_t cap = std::max(n2, std::min(std::max(held, FIRST), LIMIT - std::min(held, LIMIT)));
+      if (held + cap > LIMIT && !chunks.empty()) {
+        AMR_CUDA(cudaStreamSynchronize(s));
+        reset();
+        size_t n = 0;
+        for (; n < chunks.size() && held + cap > LIMIT; ++n) {
+          held -= chunks[n].cap;
+          cudaFreeHost(chunks[n].h);
+        }
+        chunks.erase(chunks.begin(), chunks.begin() + n);
+      }
       char* h = nullptr;
       AMR_CUDA(cudaMallocHost((void**)&h, cap));
       chunks.push_back(Chunk{h, cap});
       held += cap;
+      at = chunks.size() - 1;
       used = 0;
       wraps = 0;
     }
