@@ -106,6 +106,18 @@ __device__ __forceinline__ SplitRecip<T> split_recip(T a) {
   return r;
 }
 
+// x/2a, or a NaN where x is not finite (euler3d_split_sub); a within a_ok
+template <class T>
+__device__ __forceinline__ T split_quotient(T x, T a, const SplitRecip<T>& rc) {
+  using SR = SplitRange<T>;
+  if (SR::x_ok(x) || SR::zero(x)) {
+    const T q = SR::fma_(x, rc.rh, x * rc.rl);
+    return SR::fma_(SR::fma_(-q, T(2) * a, x), rc.rh, q);
+  }
+  // (0 * x is a zero, or the NaN that the terms left out of the sums give when x is not finite)
+  return x / (T(2) * a) + T(0) * x;
+}
+
 // Where the transverse flow is subsonic (un - a < 0 < un + a) the first wave moves only to
 // the minus side and the last only to the plus side: their terms of the other side are
 // zeros, and leaving a zero out of a sum that starts from +0 changes no value. Together with
@@ -121,14 +133,7 @@ __device__ __forceinline__ void euler3d_split_sub(const Roe3T<T>& R, const Split
   const T a3 = R.g1a2 * (R.euv * d[0] + un * d[mn - 1] + R.u[mt1] * d[mt1 - 1] + R.u[mt2] * d[mt2 - 1] - d[4]);
   const T x = d[mn - 1] + (a - un) * d[0] - a * a3;
   const T s0 = un - a, s2 = un + a;
-  T a5;
-  if (SR::x_ok(x) || SR::zero(x)) {
-    const T q = SR::fma_(x, rc.rh, x * rc.rl);
-    a5 = SR::fma_(SR::fma_(-q, T(2) * a, x), rc.rh, q);
-  } else {
-    // (0 * x is a zero, or the NaN that the terms left out below give when x is not finite)
-    a5 = x / (T(2) * a) + T(0) * x;
-  }
+  const T a5 = split_quotient(x, a, rc);
   const T a1 = d[0] - a3 - a5;
   const T a2 = d[mt1 - 1] - R.u[mt1] * d[0];
   const T a4 = d[mt2 - 1] - R.u[mt2] * d[0];
