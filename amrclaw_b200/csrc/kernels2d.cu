@@ -1467,12 +1467,9 @@ __global__ void zero_tiny_kernel(T* pool, const PatchDev* patches, const int* pl
     if (fabs((double)v) < 1e-90) v = (T)0;
   }
 }
-// Blocks of 128 threads for a patch of `items` elementwise items: four items a thread. (Eight
-// blocks a patch, whatever its size, took 2.1 ms to gather a 1002^2 Euler level's frame.)
-static int patch_blocks(long long items) { return (int)std::max<long long>(1, std::min<long long>((items + 511) / 512, 4096)); }
 void launch_zero_tiny(void* pool, const PatchDev* patches, const int* plist, int np, long long max_cells, int nvar, cudaStream_t s,
                       bool f32) {
-  const int bx = patch_blocks(max_cells * nvar);
+  const int bx = patch_blocks(max_cells * nvar, 512, np);  // four values a thread
   for (int base = 0; base < np; base += 65535) {
     const int n = std::min(65535, np - base);
     if (f32) zero_tiny_kernel<<<dim3(bx, n), 128, 0, s>>>(static_cast<float*>(pool), patches, plist + base, nvar);
@@ -1521,7 +1518,7 @@ __global__ void gather_interior2_kernel(const T* pool, const PatchDev* patches, 
 }
 void launch_gather_interior2(const void* pool, const PatchDev* patches, const int* plist, const long long* outoff,
                              int np, long long max_cells, int nvar, double* out, cudaStream_t s, bool f32) {
-  const int bx = patch_blocks(max_cells * nvar);
+  const int bx = patch_blocks(max_cells * nvar, 512, np);
   for (int base = 0; base < np; base += 65535) {
     const int n = std::min(65535, np - base);
     if (f32)

@@ -1645,7 +1645,7 @@ __global__ void zero_tiny3_kernel(T* pool, const PatchDev* patches, const int* p
 void launch_zero_tiny3(void* pool, const PatchDev* patches, const int* plist, int np, long long max_cells, int nvar, cudaStream_t s,
                        bool f32, bool aux) {
   // four values a thread (eight blocks a patch took 0.3 ms a level for patches of 64^3)
-  const int bx = (int)std::max<long long>(1, std::min<long long>((max_cells * nvar + 1023) / 1024, 4096));
+  const int bx = patch_blocks(max_cells * nvar, 1024, np);
   for (int base = 0; base < np; base += 65535) {
     const int cnt = std::min(65535, np - base);
     if (f32) zero_tiny3_kernel<<<dim3(bx, cnt), 256, 0, s>>>(static_cast<float*>(pool), patches, plist + base, cnt, nvar, aux);
