@@ -74,14 +74,15 @@ __host__ __device__ constexpr int stage_row() {
 // A tile's time is the latency of that chain, and a level of an adaptive run has fewer tiles
 // than the chip has SMs: 256 threads over chunks of six lines (114 faces) ran the chain six
 // times, solved each interface's Roe average again for its splits, and took 62 us a launch on
-// the 600 substeps of a 100^2 quadrants run; one round of 352 threads takes 27 us, and 20 us
+// the 600 substeps of a 100^2 quadrants run; one round of 352 threads takes 27 us, and 22 us
 // became 13 us for the mapped-grid advection. A uniform 1002^2 Euler level (3969 tiles) went
-// from 0.87 to 0.45 ms (one B200).
-// Waves of a face that the shared array holds at once: all of them, unless a double tile of
-// `rest` elements and `per_wave` more for each wave then takes more shared memory than a block
-// may have; the limiter goes through the waves in groups then (`least`: what the array has
-// for other uses anyway). All waves of every plugin here fit; a split step of 8 equations and
-// 5 waves, say, takes 246 KB with all of them and 222 KB with four.
+// from 0.87 to 0.43 ms (one B200).
+
+// Waves of a face that the shared array holds at once: all of them, unless a tile in doubles,
+// with `rest` values besides and `per_wave` for each wave, then takes more shared memory than a
+// block may have; the limiter goes through the waves in groups then. `least`: the values that
+// the array has for its other use. All waves of every plugin here fit; a split step of 8
+// equations and 5 waves takes 246 KB with all of them and 222 KB with four at a time.
 constexpr int wave_group(int waves, int per_wave, int least, int rest) {
   int g = waves;
   while (g > 1 && rest + (g * per_wave > least ? g * per_wave : least) > (232448 - 1024) / 8) --g;
@@ -534,10 +535,12 @@ __device__ __forceinline__ bool step2_tile(const StepArgs& a, const StepWork& wk
 }
 
 // Resident tiles per SM that the register budget is sized for. Two tiles leave a thread 80
-// registers. A thread holds the waves of its face: up to 64 bytes of them (FP32 Euler, which
-// spills 108 bytes) two tiles fit; FP64 Euler, with 128, spills 860 bytes and takes 41 us
-// instead of 30 us for a level of some 60-120 tiles (24.3 against 18.1 ms over the 600
-// substeps of a 100^2 quadrants run), and gains nothing on a level of 3969 tiles.
+// registers. A thread holds the waves of its face. Up to 64 bytes of them two tiles are better,
+// although FP32 Euler then spills 108 bytes and FP64 acoustics 80: a step of a uniform 1002^2
+// level takes 264 us against 350 with one tile for FP32 Euler, 207 against 287 for FP64 and
+// 178 against 265 for FP32 acoustics, and no adaptive run is slower. FP64 Euler, with 128 bytes,
+// spills 860 and takes 41 us instead of 30 us for a level of some 60-120 tiles (24.3 against
+// 18.1 ms over the 600 substeps of a 100^2 quadrants run), and gains nothing on 3969 tiles.
 template <class S, class R>
 constexpr int step2_blocks() {
   return S::MWAVES * S::MEQN * (int)sizeof(R) <= 64 ? 2 : 1;

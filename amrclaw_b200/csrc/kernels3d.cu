@@ -95,7 +95,7 @@ constexpr int SW_OWN = SW_T - 3;
 #define SW_MINB 3  // resident tiles per SM the register budget is sized for (FP64)
 #endif
 #ifndef SW_MINB_F32
-#define SW_MINB_F32 5  // the same for the FP32 form: half the shared buffer, 96 registers, no spills
+#define SW_MINB_F32 5  // the same for the FP32 form: half the shared buffer, 96 registers, 4 bytes of spills
 #endif
 template <class T>
 constexpr int sweep_min_blocks() { return sizeof(T) == 4 ? SW_MINB_F32 : SW_MINB; }
@@ -1475,7 +1475,9 @@ static void set_sweep_smem() {
 // direction has a third of the code (and FP64 fewer spills). 10 steps of a uniform level with
 // the frame read back, one launch against three: FP64 16^3 846 / 1129 us, 32^3 (972 tiles)
 // 1495 / 1526, 36^3 (1353) 2105 / 2031, 48^3 3146 / 2964; FP32 16^3 825 / 951, 36^3 1176 /
-// 1282, 48^3 (3063) 2147 / 2004. (Streams of their own for y and z, joined before the gather:
+// 1282, 48^3 (3063) 2147 / 2004. The swirl's sweeps have a tenth of the arithmetic and the same
+// line serves: a step in one launch / three, FP64 16^3 70 / 79 us, 32^3 84 / 90, 40^3 (1845) 98 /
+// 98; FP32 16^3 65 / 78, 32^3 73 / 85, 40^3 92 / 92, 64^3 140 / 140. (Streams of their own for y and z, joined before the gather:
 // 16^3 987 us, and nothing gained from 48^3 on.)
 template <class T>
 constexpr unsigned merge_tiles() { return 148u * (unsigned)sweep_min_blocks<T>() * 9u / 4u; }
