@@ -1461,24 +1461,29 @@ template <class T, class PH>
 static void set_sweep_smem() {
   static const bool done = [] {
     constexpr int smem = sweep3_smem_bytes<T, PH>();
-    AMR_CUDA(cudaFuncSetAttribute(sweep3_kernel<1, T, PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    AMR_CUDA(cudaFuncSetAttribute(sweep3_kernel<2, T, PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    AMR_CUDA(cudaFuncSetAttribute(sweep3_kernel<3, T, PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     AMR_CUDA(cudaFuncSetAttribute(sweep3_all_kernel<T, PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if constexpr (HasQuick<PH>::value) {
+      AMR_CUDA(cudaFuncSetAttribute(sweep3_kernel<1, T, PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      AMR_CUDA(cudaFuncSetAttribute(sweep3_kernel<2, T, PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      AMR_CUDA(cudaFuncSetAttribute(sweep3_kernel<3, T, PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    }
     return true;
   }();
   (void)done;
 }
-// Tiles up to which the three directions go in one launch: nine quarters of the blocks that
+// Tiles up to which the three directions of a plugin with a quick form, whose kernels hold its
+// splits twice for each direction, go in one launch: nine quarters of the blocks that
 // are resident at once (148 SMs). A level below that leaves SMs idle in launches of its own,
 // one direction after another; above it the last wave matters less than that a kernel of one
 // direction has a third of the code (and FP64 fewer spills). 10 steps of a uniform level with
 // the frame read back, one launch against three: FP64 16^3 846 / 1129 us, 32^3 (972 tiles)
 // 1495 / 1526, 36^3 (1353) 2105 / 2031, 48^3 3146 / 2964; FP32 16^3 825 / 951, 36^3 1176 /
-// 1282, 48^3 (3063) 2147 / 2004. The swirl's sweeps have a tenth of the arithmetic and the same
-// line serves: a step in one launch / three, FP64 16^3 70 / 79 us, 32^3 84 / 90, 40^3 (1845) 98 /
-// 98; FP32 16^3 65 / 78, 32^3 73 / 85, 40^3 92 / 92, 64^3 140 / 140. (Streams of their own for y and z, joined before the gather:
+// 1282, 48^3 (3063) 2147 / 2004. (Streams of their own for y and z, joined before the gather:
 // 16^3 987 us, and nothing gained from 48^3 on.)
+// A plugin without a quick form takes one launch at every size: nothing spills, and the last
+// waves of two launches are saved. A step of the swirl in one launch / three / three on streams
+// of their own: FP64 16^3 70 / 79 / 79 us, 40^3 96 / 101 / 94, 64^3 172 / 181 / 179, 96^3 397 /
+// 415 / 420; FP32 16^3 65 / 78 / 72, 40^3 84 / 92 / 78, 64^3 125 / 140 / 126, 96^3 286 / 303 / 299.
 template <class T>
 constexpr unsigned merge_tiles() { return 148u * (unsigned)sweep_min_blocks<T>() * 9u / 4u; }
 // the three sweep directions of a level, in one launch or one each
@@ -1489,13 +1494,15 @@ static int launch_sweeps(const Step3Args& a, const long long items[3], cudaStrea
   set_sweep_smem<T, PH>();
   int n = 0;
   const unsigned nx = tiles(items[0]), nxy = nx + tiles(items[1]), nall = nxy + tiles(items[2]);
-  if (nall <= merge_tiles<T>()) {
+  if (!HasQuick<PH>::value || nall <= merge_tiles<T>()) {
     if (nall > 0) { sweep3_all_kernel<T, PH><<<nall, SW_T, smem, s>>>(a, nx, nxy); ++n; }
     return n;
   }
-  if (items[0] > 0) { sweep3_kernel<1, T, PH><<<tiles(items[0]), SW_T, smem, s>>>(a); ++n; }
-  if (items[1] > 0) { sweep3_kernel<2, T, PH><<<tiles(items[1]), SW_T, smem, s>>>(a); ++n; }
-  if (items[2] > 0) { sweep3_kernel<3, T, PH><<<tiles(items[2]), SW_T, smem, s>>>(a); ++n; }
+  if constexpr (HasQuick<PH>::value) {
+    if (items[0] > 0) { sweep3_kernel<1, T, PH><<<tiles(items[0]), SW_T, smem, s>>>(a); ++n; }
+    if (items[1] > 0) { sweep3_kernel<2, T, PH><<<tiles(items[1]), SW_T, smem, s>>>(a); ++n; }
+    if (items[2] > 0) { sweep3_kernel<3, T, PH><<<tiles(items[2]), SW_T, smem, s>>>(a); ++n; }
+  }
   return n;
 }
 template <class T, class PH>
