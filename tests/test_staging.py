@@ -55,7 +55,8 @@ def lib(tmp_path_factory):
     with open(d + "/staging.cpp", "w") as f:
         f.write(SRC)
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc()))), "include")
-    subprocess.run(["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-I", CSRC, "-I", cuda, "-o", d + "/staging.so",
+    # (bound to the stand-ins here, also where the process has loaded a CUDA runtime)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", CSRC, "-I", cuda, "-o", d + "/staging.so",
                     d + "/staging.cpp"], check=True)
     lib = ctypes.CDLL(d + "/staging.so")
     lib.stage.restype = ctypes.c_longlong
@@ -90,7 +91,7 @@ def test_an_upload_past_the_limit_is_alone(lib):
 
 def test_small_uploads_grow_with_use(lib):
     held, syncs = run(lib, [300_000] * 2000, wait_every=10)
-    assert max(held) <= 8 * MB and syncs == 200  # a round of 3 MB fits: only the caller waits
+    assert max(held) <= 8 * MB and syncs == 200  # ten of them fit: only the caller waits
     held, syncs = run(lib, [3 * MB] * 400, soon=32 * MB)
     assert held[-1] <= LIMIT and syncs < 60
     assert held == sorted(held)
