@@ -68,7 +68,8 @@ int amrgpu_set_graphs(amrgpu_ctx* ctx, int on);
 int amrgpu_checkpoint(amrgpu_ctx* ctx, const char* path);
 
 /* Sweep schedule of the batched 3D path. 1 (default): one launch per sweep direction (a
- * block per tile of 128 interfaces); 2: one persistent work-queue launch in which resident
+ * block per tile of 128 interfaces; small levels, and solvers with one form of their splits,
+ * take the three directions in one); 2: one persistent work-queue launch in which resident
  * blocks take the tiles of all three directions from an atomic counter; 0: autotune per
  * level (the level's first substeps alternate the two, timed with CUDA events per
  * cell-update, and the faster is kept). Results are identical under every schedule.
