@@ -273,7 +273,7 @@ class Amr2Gpu {
     if (prob.solver == SOLVER_VC_ADVECTION && p.naux < VcAdvection2::NAUX)
       throw std::runtime_error("vc_advection reads aux(1) and aux(2): num_aux must be at least 2");
     sp.prob = prob;
-    for (int k = 0; k < MAXVAR; ++k) sp.mthlim[k] = k < (int)p.mthlim.size() ? p.mthlim[k] : 0;
+    for (int k = 0; k < MAXWAVE; ++k) sp.mthlim[k] = k < (int)p.mthlim.size() ? p.mthlim[k] : 0;
     sp.order = p.order; sp.trans = p.trans; sp.use_fwaves = p.use_fwaves ? 1 : 0; sp.mcapa = p.mcapa;
     sp.split = p.dimsplit;
   }

@@ -298,7 +298,7 @@ class Amr3Gpu : public AmrSolver {
     xperdom = p.mthbc[1] == 2; yperdom = p.mthbc[3] == 2; zperdom = p.mthbc[5] == 2;
     sp.gamma = p.pn("gamma", 1.4); sp.gamma1 = sp.gamma - 1.0;
     sp.efix = (int)p.pn("efix", 1.0);
-    for (int k = 0; k < 3; ++k) sp.mthlim[k] = k < (int)p.mthlim.size() ? p.mthlim[k] : 0;
+    for (int k = 0; k < MAXWAVE; ++k) sp.mthlim[k] = k < (int)p.mthlim.size() ? p.mthlim[k] : 0;
     sp.order = p.order;
     if (p.trans < 0) throw std::runtime_error("transverse_waves < 0 is not supported");
     sp.m3 = p.trans / 10; sp.m4 = p.trans - 10 * sp.m3;

@@ -17,7 +17,7 @@
 namespace amrb {
 
 constexpr int MAXLV = 10;
-constexpr int MAXVAR = 5;
+constexpr int MAXWAVE = 12;  // waves a plugin may have (the step parameters hold a limiter for each)
 
 // Flag values of the reference (src/2d/amr_module.f90:163-168), stored as int8 codes.
 constexpr int8_t FLAG_UNSET = -1, FLAG_DONT = 0, FLAG_DO = 2, FLAG_BADPRO = 3;

@@ -92,6 +92,7 @@ constexpr int wave_group(int waves, int per_wave, int least, int rest) {
 template <class S>
 struct Step2Layout {
   static constexpr int ME = S::MEQN, MW = S::MWAVES;
+  static_assert(MW <= MAXWAVE, "StepParams holds a limiter for every wave");
   static constexpr int T = TILE2;
   static constexpr int QW = T + 4;
   static constexpr int NLINE = T + 2, NFACE = T + 3;
@@ -627,6 +628,7 @@ __global__ void __launch_bounds__(STEP2_THREADS, step2_blocks<S, R>()) step2_bat
 template <class S>
 struct Split2Layout {
   static constexpr int ME = S::MEQN, MW = S::MWAVES, T = TILE2, QW = T + 4, NFACE = T + 3;
+  static_assert(MW <= MAXWAVE, "StepParams holds a limiter for every wave");
   static constexpr int PITCH = QW * NFACE;          // elements of one shared wave value over the faces
   static constexpr int NQ = ME * QW * QW;           // staged q of the tile and two ghost layers
   static constexpr int NFX = ME * QW * (T + 1);      // fm / fp of every staged row

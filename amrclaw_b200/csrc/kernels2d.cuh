@@ -34,7 +34,7 @@ struct FadEntry {
 
 struct StepParams {
   ProbDev prob;
-  int mthlim[MAXVAR];
+  int mthlim[MAXWAVE];
   int order;             // method(2)
   int trans;             // method(3)
   int use_fwaves;

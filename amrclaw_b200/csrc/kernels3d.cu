@@ -352,6 +352,7 @@ __device__ __forceinline__ void trans_side(const PH& ph, int imp, const T* F, co
 template <int DIR, class T, class PH, bool QUICK = HasQuick<PH>::value>
 __device__ __forceinline__ void sweep3_tile(const Step3Args& A, long long tile, T (*sW)[SW_T]) {
   constexpr int NV = PH::NV, NW = PH::NW;
+  static_assert(NW <= MAXWAVE, "Step3Params holds a limiter for every wave");
   T* const sG = &sW[0][0];
   auto G = [&](int x, int col) -> T& { return sG[x * SW_T + col]; };
   const long long* c0 = A.comp0 + (long long)(DIR - 1) * (A.np + 1);
@@ -541,6 +542,7 @@ __global__ void __launch_bounds__(SW_T, sweep_min_blocks<T>()) sweep3_queue_kern
 template <int DIR, class T, class PH>
 __global__ void __launch_bounds__(SW_T) split3_kernel(Step3Args A) {
   constexpr int NV = PH::NV, NW = PH::NW;
+  static_assert(NW <= MAXWAVE, "Step3Params holds a limiter for every wave");
   __shared__ T sW[NW * NV][SW_T];
   __shared__ T sF[2 * NV][SW_T];
   const long long* c0 = A.scomp0 + (long long)(DIR - 1) * (A.np + 1);

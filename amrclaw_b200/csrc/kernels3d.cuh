@@ -31,7 +31,7 @@ struct Step3Params {
   int solver;  // Solver3
   double gamma, gamma1;
   int efix;
-  int mthlim[3];
+  int mthlim[MAXWAVE];
   int order;   // method(2)
   int m3, m4;  // method(3) = 10*m3 + m4
 };

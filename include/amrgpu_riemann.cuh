@@ -13,7 +13,7 @@
  * name and sets its constants (the reference's /cparam/ common block).
  *
  * 2D plugin (a struct S; R is float or double; P is the constants struct):
- *   static constexpr int MEQN, MWAVES, NAUX;
+ *   static constexpr int MEQN, MWAVES (at most 12), NAUX;
  *   __device__ static void rpn(const P&, int ixy, const R* qL, const R* qR,
  *                              const R* auxL, const R* auxR,
  *                              R (&wave)[MWAVES][MEQN], R (&s)[MWAVES],
@@ -30,7 +30,7 @@
  *   be null).
  *
  * 3D plugin (a struct S<R> holding the interface's per-call state):
- *   static constexpr int NV (meqn), NW (mwaves);
+ *   static constexpr int NV (meqn), NW (mwaves, at most 12);
  *   template <int DIR> __device__ void load(pool, patch, base, step, plane, e);
  *       reads the aux values the interface needs (nothing for Euler);
  *   template <int DIR> __device__ void rpn(const Step3Params&, const R* QL, const R* QR,

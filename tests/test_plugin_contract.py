@@ -28,6 +28,8 @@ struct Contract3 {
 };
 static_assert(amrgpu_plugin::Check3D<Contract3<double>, Step3Params, double>::value, "");
 static_assert(amrgpu_plugin::Check3D<Contract3<float>, Step3Params, float>::value, "");
+// a limiter for each wave of a larger plugin
+static_assert(sizeof(Step3Params::mthlim) / sizeof(int) >= 8, "");
 template int launch_step3_t<double, Contract3<double>>(const Step3Args&, const long long*, long long, long long, cudaStream_t);
 template int launch_step3_t<float, Contract3<float>>(const Step3Args&, const long long*, long long, long long, cudaStream_t);
 }
@@ -59,6 +61,8 @@ static_assert(split_fits<Contract2<7, 7>>() && split_fits<Contract2<8, 7>>() && 
 static_assert(split_fits<Contract2<11, 3>>() && split_fits<Contract2<12, 1>>(), "");
 // the plugins of this library have all their waves there at once
 static_assert(Step2Layout<Euler2>::WG == 4 && Split2Layout<Euler2>::WG == 4 && Split2Layout<Acoustics2>::WG == 2, "");
+// a limiter for each wave of a larger plugin
+static_assert(sizeof(StepParams::mthlim) / sizeof(int) >= 8, "");
 static_assert(amrgpu_plugin::Check2D<Contract2<8, 5>, ProbDev, double>::value, "");
 template void launch_step2_t<Contract2<8, 5>, double>(const StepArgs&, int, cudaStream_t);
 template void launch_step2_t<Contract2<8, 5>, float>(const StepArgs&, int, cudaStream_t);

@@ -1,6 +1,6 @@
 """The 2D step of plugins whose waves do not all fit in shared memory at once: five waves that
-each carry two of ten components give every pair of components what a plugin with that one
-wave alone gives it, in the unsplit and the split step, order 1 and 2."""
+each carry two of ten components (in FP32 seven, of fourteen) give every pair of components what
+a plugin with that one wave alone gives it, in the unsplit and the split step, order 1 and 2."""
 import ctypes
 import subprocess
 
@@ -80,17 +80,23 @@ static int step(R* q, int mx, int my, int order, int trans, int split) {
   } catch (std::exception& e) { std::fprintf(stderr, "%s\\n", e.what()); return 1; }
   return 0;
 }
-template <int W>
-static int one(double* q, int mx, int my, int order, int trans, int split, int k) {
-  if (k == W) return step<Pairs<1, W>, double>(q, mx, my, order, trans, split);
-  if constexpr (W < 4) return one<W + 1>(q, mx, my, order, trans, split, k);
+template <int W, int N, class R>
+static int one(R* q, int mx, int my, int order, int trans, int split, int k) {
+  if (k == W) return step<Pairs<1, W>, R>(q, mx, my, order, trans, split);
+  if constexpr (W + 1 < N) return one<W + 1, N>(q, mx, my, order, trans, split, k);
   return 2;
 }
-extern "C" int run_five(double* q, int mx, int my, int order, int trans, int split) {
+extern "C" int run_all64(double* q, int mx, int my, int order, int trans, int split) {
   return step<Pairs<5, 0>, double>(q, mx, my, order, trans, split);
 }
-extern "C" int run_one(double* q, int mx, int my, int order, int trans, int split, int k) {
-  return one<0>(q, mx, my, order, trans, split, k);
+extern "C" int run_one64(double* q, int mx, int my, int order, int trans, int split, int k) {
+  return one<0, 5>(q, mx, my, order, trans, split, k);
+}
+extern "C" int run_all32(float* q, int mx, int my, int order, int trans, int split) {
+  return step<Pairs<7, 0>, float>(q, mx, my, order, trans, split);
+}
+extern "C" int run_one32(float* q, int mx, int my, int order, int trans, int split, int k) {
+  return one<0, 7>(q, mx, my, order, trans, split, k);
 }
 }
 """
@@ -106,16 +112,18 @@ def lib(tmp_path_factory):
     return ctypes.CDLL(d + "/waves.so")
 
 
+@pytest.mark.parametrize("bits,waves", [(64, 5), (32, 7)])
 @pytest.mark.parametrize("mx,my", [(1, 1), (16, 16), (17, 15), (40, 37)])
 @pytest.mark.parametrize("order,trans,split", [(2, 2, 0), (2, 1, 0), (1, 0, 0), (2, 0, 1), (1, 0, 1)])
-def test_pairs_of_components(lib, mx, my, order, trans, split):
-    p = lambda a: a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
-    q = np.random.default_rng(mx + my).normal(size=(10, my + 4, mx + 4))
-    all5 = q.copy()
-    assert lib.run_five(p(all5), mx, my, order, trans, split) == 0
+def test_pairs_of_components(lib, mx, my, order, trans, split, bits, waves):
+    run_all, run_one = (lib.run_all64, lib.run_one64) if bits == 64 else (lib.run_all32, lib.run_one32)
+    p = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    q = np.random.default_rng(mx + my).normal(size=(2 * waves, my + 4, mx + 4)).astype("f%d" % (bits // 8))
+    together = q.copy()
+    assert run_all(p(together), mx, my, order, trans, split) == 0
     inside = (slice(None), slice(2, my + 2), slice(2, mx + 2))
-    assert not np.array_equal(all5[inside], q[inside])
-    for k in range(5):
+    assert not np.array_equal(together[inside], q[inside])
+    for k in range(waves):
         pair = np.ascontiguousarray(q[2 * k:2 * k + 2])
-        assert lib.run_one(p(pair), mx, my, order, trans, split, k) == 0
-        assert np.array_equal(pair[inside], all5[2 * k:2 * k + 2][inside]), k
+        assert run_one(p(pair), mx, my, order, trans, split, k) == 0
+        assert np.array_equal(pair[inside], together[2 * k:2 * k + 2][inside]), k
